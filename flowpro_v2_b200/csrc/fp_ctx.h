@@ -105,15 +105,15 @@ struct fp_ctx {
     unsigned ilu_epoch = 0;          // epoch of the last application
     unsigned ilu_fepoch = 0;         // epoch of the last factorisation
     int ilu_max_polls = 1 << 19;     // poll limit of every dependency wait of the ILU kernels
-    unsigned long long* d_ilu_pub = nullptr;  // [2][nElem][nc][2] published sweep values (forward, backward)
+    unsigned long long* d_ilu_pub = nullptr;  // [4 nElem nc] published sweep values (forward, backward; two words each, or two halves)
     int sweep_grid = 0;           // thread blocks of the persistent sweep kernel
-    // bulk-copy sweep kernel per factor precision [FP64, FP32]: slots, grid (-1 unknown, 0 not
-    // applicable), dynamic shared memory
-    int sweep_bulk_S[2] = {0, 0};
-    int sweep_bulk_NG[2] = {0, 0};   // positions in flight per block (0: not tuned yet)
-    int sweep_bulk_grid[2] = {-1, -1};
-    size_t sweep_bulk_smem[2] = {0, 0};
-    int sweep_variant = 0;           // 0 bulk-copy staged (autotuned groups), 1 register, 2-6 bulk with 1-16 groups
+    // streamed sweep kernel per factor precision [FP64, FP32]: grid (0: not configured yet) and
+    // blocks of its shared-memory ring; whether d_ilu_pub holds its words, and which half is next
+    int ring_grid[2] = {0, 0};
+    int ring_blocks[2] = {0, 0};
+    bool ring_pub_ready = false;
+    int ring_parity = 0;
+    int sweep_variant = 0;           // 0 streamed, 1 register, 2-6 streamed with 1-16 elements in flight per block
     // Krylov
     int kry_m = 0;
     bool kry_transposed = false;  // GMRES on A^T (adjoint solves)
@@ -233,6 +233,8 @@ int ilu_factor(fp_ctx* c, int precision);                        // block ILU(0)
 int ilu_prepare_direct(fp_ctx* c, int precision, void** F);      // factor storage for blocks written in place
 int ilu_factor_direct(fp_ctx* c, int precision);                 // factorise the blocks written in place
 int ilu_apply(fp_ctx* c, const double* x, double* y);
+bool ring_sweep_applies(int nc);                                 // fp_ilu_ring.cu
+int ring_sweep(fp_ctx* c, int precision, const double* b, double* x, int groups);  // groups 0: all
 int ilu_check(fp_ctx* c);                                        // FP_ERR_TIMEOUT if a sweep wait gave up
 void ilu_release(fp_ctx* c);
 int gmres(fp_ctx* c, int jacobian, int kind, int restart, int max_restarts, double tol, int* iters, double* rel);

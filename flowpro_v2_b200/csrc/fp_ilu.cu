@@ -20,10 +20,11 @@
 //     (bounded) only for the completion flags of its lower neighbours;
 //   * an application (forward L sweep, backward U sweep) is ONE persistent cooperative
 //     kernel: thread blocks take the elements in level order, and each element waits
-//     (bounded) only for the values of the neighbours it multiplies, which are published
-//     with the epoch of the application in every word, so levels overlap and no flag or
-//     fence stands between a value and its consumer.  Each element's factor blocks are
-//     loaded into registers before the values they multiply arrive;
+//     (bounded) only for the values of the neighbours it multiplies, so levels overlap and no
+//     flag or fence stands between a value and its consumer.  Even numbers of unknowns take
+//     fp_ilu_ring.cu, which streams the factor blocks through shared memory; the kernel here
+//     (odd numbers, or on request) loads each element's factor entries into registers before
+//     the values they multiply arrive, and its words carry the epoch of the application;
 //   * the factorisation runs in the precision of the factors: FP64, or FP32 for the
 //     mixed-precision GMRES, where the blocks are either gathered from the assembled
 //     operator (rounded) or written straight into the FP32 factor storage by the exact
@@ -517,271 +518,6 @@ __global__ void __launch_bounds__(kSweepThreads)
     }
 }
 
-// ---------------------------------------------------------------------------- bulk-copy sweeps
-// The same application with the factor blocks staged in shared memory by bulk asynchronous
-// copies (the TMA engine's cp.async.bulk, one instruction per block, completion counted in
-// bytes on an mbarrier) up to S positions ahead.  An element's blocks are contiguous in the
-// element-major factor storage (F[e][s], nc * nc values each), so thread 0 requests exactly the
-// blocks the position multiplies (forward: the lower neighbours' L blocks; backward: the upper
-// neighbours' U blocks and inv(U_ii)) into slot k % S and the block's threads read them from
-// shared memory when the position's turn comes.  A slot is refilled as soon as the barrier of
-// the next position shows every thread done with it, and the program entries are loaded a
-// position ahead, so one barrier per forward position (two backward) is on the path.  One block per SM holds S slots of (1 + nf)
-// blocks; the per-position arithmetic is the register kernel's, in the same order, so both give
-// identical results.  Needs nc * nc * sizeof(T) to be a multiple of 16 bytes (bulk-copy size and
-// address alignment).
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-    unsigned ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_addr(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// global -> shared bulk copy of `bytes` (multiple of 16, both addresses 16-byte aligned),
-// completing on bar; no cluster multicast
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
-constexpr int kBulkPolls = 1 << 22;  // a bulk copy from device memory completes within microseconds
-
-// Bounded wait for phase `parity` of bar.  A wait that runs out sets FP_DEV_TIMEOUT and the
-// abort word and returns false.
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity, unsigned* abortw, unsigned* status) {
-    for (int it = 0; it < kBulkPolls; it++)
-        if (mbar_try_wait(bar, parity)) return true;
-    atomicOr(status, (unsigned)FP_DEV_TIMEOUT);
-    atomicExch(abortw, 1u);
-    return false;
-}
-
-// thread 0: request the blocks the position of element i with neighbours nbv multiplies into
-// slot (forward: the neighbours' blocks 1 + f; backward: those and block 0)
-// (skip: an arrival without bytes, which completes the slot's phase at once)
-template <class T>
-__device__ __forceinline__ void sweep_request(bool bwd, int i, int4 nbv, int nc2, int nf, const T* __restrict__ F, T* slot,
-                                              unsigned long long* bar, bool skip) {
-    if (skip) {
-        mbar_expect_tx(bar, 0u);
-        return;
-    }
-    const int nb[kMaxF] = {nbv.x, nbv.y, nbv.z, nbv.w};
-    const unsigned bb = (unsigned)(nc2 * sizeof(T));
-    unsigned bytes = bwd ? bb : 0u;
-    for (int f = 0; f < nf; f++)
-        if (nb[f] >= 0) bytes += bb;
-    mbar_expect_tx(bar, bytes);
-    const T* src = F + (size_t)i * (1 + nf) * nc2;
-    if (bwd) bulk_load(slot, src, bb, bar);
-    for (int f = 0; f < nf; f++)
-        if (nb[f] >= 0) bulk_load(slot + (size_t)(1 + f) * nc2, src + (size_t)(1 + f) * nc2, bb, bar);
-}
-
-// barrier of the threads of group grp: a warp-wide sync for one-warp groups, else named
-// barrier 1 + grp (ids 1 .. 8; 0 is __syncthreads)
-__device__ __forceinline__ void group_sync(int grp, int nthreads) {
-    if (nthreads == 32)
-        __syncwarp();
-    else
-        asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(nthreads) : "memory");
-}
-
-// Most groups per block of the staged sweep for nc unknowns per element (16 one-warp groups
-// for nc <= 16, 8 for nc <= 32, else 4), and the lanes per row that go with it: a power of two,
-// adjacent in one warp, such that a row set fits a group of the most groups.  The lane split
-// depends on nc alone, so the sums, and the results, do not depend on the group count.  It is
-// at least 2 for every nc up to kMaxNc: lanes 0 and 1 of a row publish the two halves of its
-// value.
-constexpr __host__ __device__ int sweep_max_groups(int nc) { return nc <= 16 ? 16 : nc <= 32 ? 8 : 4; }
-constexpr __host__ __device__ int sweep_row_lanes(int nc) {
-    const int lim = kSweepThreads / sweep_max_groups(nc);
-    int G = 32;
-    while (G > 1 && G * nc > lim) G >>= 1;
-    return G;
-}
-constexpr bool sweep_lanes_publish(int nc) { return nc > kMaxNc || (sweep_row_lanes(nc) >= 2 && sweep_lanes_publish(nc + 1)); }
-static_assert(sweep_lanes_publish(1), "every row of the staged sweep needs two lanes up to kMaxNc unknowns");
-
-// k-th position of this block's sequence: forward b, b + GB, ... (< nE), then backward
-// nE + b, nE + b + GB, ... (GB = gridDim.x); nV past the end
-__device__ __forceinline__ int block_position(int k, int nE) {
-    const int b = (int)blockIdx.x, GB = (int)gridDim.x;
-    const int Jf = b < nE ? (nE - 1 - b) / GB + 1 : 0;
-    if (k < Jf) return b + k * GB;
-    const int v = nE + b + (k - Jf) * GB;
-    return v < 2 * nE ? v : 2 * nE;
-}
-
-// The block's 512 threads form NG groups of 512 / NG threads; group g takes the positions
-// k = g, g + NG, ... of the block's sequence, so NG positions are in flight per block, each
-// group synchronising on its own barrier.  Slot k % S holds position k's factor blocks;
-// S is a multiple of NG, so a slot always serves the same group, whose leader refills it with
-// position k + S as soon as the group is done with position k.  With live flags (batched cases:
-// caseOf, live non-null), the positions of a case whose flag is 0 only keep the slot rotation
-// (no copy, no wait on neighbours, no value published); no position of another case depends on
-// them.  Dynamic shared memory: the
-// S slots, their S mbarriers, then per group (of sweep_max_groups(nc)) the neighbours' values
-// (nf * nc), the element's forward value and its value before inv(U_ii) (nc each).
-template <class T>
-__global__ void __launch_bounds__(kSweepThreads, 2)
-    k_ilu_sweeps_bulk(int nc, int nf, int ld, int nE, int S, int NG, const int* __restrict__ swEl,
-                      const int4* __restrict__ swNb, const T* __restrict__ F, const double* __restrict__ b,
-                      double* __restrict__ x, unsigned long long* pubF, unsigned long long* pubB, unsigned epoch,
-                      unsigned* abortw, unsigned* status, int maxPolls, const int* __restrict__ caseOf,
-                      const int* __restrict__ live) {
-    extern __shared__ __align__(128) unsigned char sweep_smem[];
-    const int nc2 = nc * nc, ns = 1 + nf;
-    T* slots = reinterpret_cast<T*>(sweep_smem);
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(sweep_smem + (size_t)S * ns * nc2 * sizeof(T));
-    __shared__ int failed[16];
-    const int GT = kSweepThreads / NG;  // threads of a group
-    const int grp = threadIdx.x / GT, t = threadIdx.x - grp * GT;
-    const int G = sweep_row_lanes(nc);
-    const int r = t / G, g = t - r * G;
-    const int nV = 2 * nE;
-    if ((int)blockIdx.x >= nE) return;
-    if (threadIdx.x == 0) {
-        for (int q = 0; q < S; q++) mbar_init(bars + q, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (t == 0) failed[grp] = 0;
-    __syncthreads();
-    double* vs = reinterpret_cast<double*>(bars + S) + (size_t)grp * (nf + 2) * nc;  // [nf][nc]
-    double* yo = vs + (size_t)nf * nc;
-    double* tv = yo + nc;
-    // the group leader requests its positions grp, grp + NG, ... below S
-    int kq = grp;  // next sequence index to request (leader)
-    if (t == 0) {
-        for (; kq < S; kq += NG) {
-            const int vq = block_position(kq, nE);
-            if (vq >= nV) break;
-            const int iq = swEl[vq];
-            sweep_request<T>(vq >= nE, iq, swNb[vq], nc2, nf, F, slots + (size_t)(kq % S) * ns * nc2, bars + kq % S,
-                             live && !live[caseOf[iq]]);
-        }
-    }
-    int k = grp;
-    int v = block_position(k, nE);
-    int i_cur = v < nV ? swEl[v] : 0;
-    int4 nb_cur = v < nV ? swNb[v] : make_int4(-1, -1, -1, -1);
-    while (v < nV) {
-        const int q = k % S;
-        const bool bwd = v >= nE;
-        const T* Fs = slots + (size_t)q * ns * nc2;
-        const int i = i_cur;
-        const int4 nbv = nb_cur;
-        const int vn = block_position(k + NG, nE);
-        if (vn < nV) {  // the group's next program entry, in flight during this position
-            i_cur = swEl[vn];
-            nb_cur = swNb[vn];
-        }
-        unsigned long long* pub = bwd ? pubB : pubF;  // the neighbours' values and this element's
-        const bool skip = live && !live[caseOf[i]];  // the same for the whole group
-        const double a_in = (!skip && !bwd && g < 2 && r < nc) ? __ldcg(b + (size_t)r * ld + i) : 0.0;  // the two publishing lanes
-        // word u: half u & 1 of value (u / 2) mod nc of neighbour f = u / (2 nc); each thread's
-        // words go four at a time, their first loads in flight together, and only a word not
-        // yet of this epoch is polled again
-        const int nw = skip ? 0 : nf * nc * 2;
-        for (int u0 = t; u0 < nw; u0 += 4 * GT) {
-            const unsigned long long* pp[4];
-            unsigned long long pv[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int u = u0 + q * GT;
-                pp[q] = nullptr;
-                if (u < nw) {
-                    const int f = u / (2 * nc), cw = u - f * 2 * nc;
-                    const int n = f == 0 ? nbv.x : f == 1 ? nbv.y : f == 2 ? nbv.z : nbv.w;
-                    if (n >= 0) pp[q] = pub + (size_t)n * nc * 2 + cw;
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++) pv[q] = pp[q] ? pub_load(pp[q]) : 0ull;
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const int u = u0 + q * GT;
-                if (u < nw) {
-                    unsigned w = 0u;
-                    if (pp[q])
-                        w = (unsigned)(pv[q] >> 32) == epoch ? (unsigned)pv[q] : pub_wait(pp[q], epoch, abortw, status, maxPolls);
-                    reinterpret_cast<unsigned*>(vs)[u] = w;
-                }
-            }
-        }
-        if (bwd && !skip)
-            for (int u = t; u < 2 * nc; u += GT)
-                reinterpret_cast<unsigned*>(yo)[u] = pub_wait(pubF + (size_t)i * nc * 2 + u, epoch, abortw, status, maxPolls);
-        // the position's factor blocks have arrived in slot q
-        if (!mbar_wait(bars + q, (unsigned)((k / S) & 1), abortw, status)) failed[grp] = 1;
-        group_sync(grp, GT);
-        if (failed[grp]) break;
-        if (!skip) {
-            const int nb[kMaxF] = {nbv.x, nbv.y, nbv.z, nbv.w};
-            double sf[kMaxF];
-#pragma unroll
-            for (int f = 0; f < kMaxF; f++) {
-                sf[f] = 0.0;
-                if (f < nf && nb[f] >= 0 && r < nc) {
-                    const T* Bf = Fs + (size_t)(1 + f) * nc2;
-                    for (int c = g; c < nc; c += G) sf[f] += (double)Bf[c * nc + r] * vs[f * nc + c];
-                }
-            }
-            const double s = group_sum((sf[0] + sf[1]) + (sf[2] + sf[3]), G);
-            double a;
-            if (!bwd) {
-                a = a_in - s;
-            } else {
-                if (g == 0 && r < nc) tv[r] = yo[r] - s;
-                group_sync(grp, GT);
-                double d = 0.0;
-                if (r < nc)
-                    for (int c = g; c < nc; c += G) d += (double)Fs[c * nc + r] * tv[c];
-                a = group_sum(d, G);
-                if (g == 0 && r < nc) x[(size_t)r * ld + i] = a;
-            }
-            if (g < 2 && r < nc) {
-                const unsigned long long e = (unsigned long long)epoch << 32;
-                pub_store(pub + ((size_t)i * nc + r) * 2 + g, e | (unsigned)(g == 0 ? __double2loint(a) : __double2hiint(a)));
-            }
-        }
-        // the group is done with slot q: it takes the group's position S ahead
-        group_sync(grp, GT);
-        if (t == 0) {
-            const int vq = block_position(kq, nE);
-            if (vq < nV) {
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                const int iq = swEl[vq];
-                sweep_request<T>(vq >= nE, iq, swNb[vq], nc2, nf, F, slots + (size_t)q * ns * nc2, bars + q,
-                                 live && !live[caseOf[iq]]);
-                kq += NG;
-            }
-        }
-        v = vn;
-        k += NG;
-    }
-    // after a failed copy wait: let the group's copies still in flight land before the block exits
-    if (t == 0 && failed[grp]) {
-        for (int kk = k; kk < kq; kk += NG) {
-            unsigned long long* bar = bars + kk % S;
-            for (int it = 0; it < kBulkPolls && !mbar_try_wait(bar, (unsigned)((kk / S) & 1)); it++) {
-            }
-        }
-    }
-}
-
 // levels, neighbour sets and the per-element factorisation program (host, once per mesh)
 int ilu_build(fp_ctx* c) {
     const HostMesh& h = c->hm;
@@ -903,6 +639,8 @@ int ilu_build(fp_ctx* c) {
     c->sweep_grid = std::max(1, std::min(nE, nsm * std::max(1, std::min(perSm, perSm32))));
     c->ilu_epoch = 0;
     c->ilu_fepoch = 0;
+    c->ring_pub_ready = false;
+    c->ring_parity = 0;
     c->ilu_built = true;
     return FP_OK;
 }
@@ -1021,7 +759,9 @@ void ilu_release(fp_ctx* c) {
     c->d_swEl = nullptr;
     c->d_ilu_pub = nullptr;
     c->sweep_grid = 0;
-    c->sweep_bulk_grid[0] = c->sweep_bulk_grid[1] = -1;
+    c->ring_grid[0] = c->ring_grid[1] = 0;
+    c->ring_pub_ready = false;
+    c->ring_parity = 0;
 
     c->lvlF_ptr.clear();
     c->lvlB_ptr.clear();
@@ -1062,139 +802,53 @@ int ilu_factor_direct(fp_ctx* c, int precision) {
     return FP_OK;
 }
 
-// bulk-copy sweep configuration of factor type T: slots per block, grid, dynamic shared
-// memory (grid 0: the register kernel is used)
-// slots per block, grid and dynamic shared memory of the bulk-copy sweep for factor type T
-// (grid 0: the register kernel is used)
+// the register kernel (odd numbers of unknowns, and fp_set_ilu_sweep(ctx, 1))
 template <class T>
-int bulk_sweep_config(fp_ctx* c, int* S_out, int* grid_out, size_t* smem_out) {
-    const size_t nc2 = (size_t)c->nc * c->nc, ns = 1 + c->hm.nf;
-    *grid_out = 0;
-    if ((nc2 * sizeof(T)) % 16 != 0 || c->nc > kSweepThreads / 4) return FP_OK;
-    if (sweep_row_lanes(c->nc) < 2) return FP_OK;  // a row's value is published by two lanes
-    const size_t slot = ns * nc2 * sizeof(T);
-    // slot budget: 208 KB (one block per SM) for large blocks, 100 KB (two blocks per SM, the
-    // register limit of __launch_bounds__) for nc <= 32
-    const size_t budget = (c->nc > 32 ? 208 : 100) * 1024;
-    int S = (int)std::min<size_t>(32, budget / slot);
-    if (S < 2) return FP_OK;
-    int p = 2;  // S: a multiple of the largest power of two up to the group limit that fits
-    while (2 * p <= std::min(S, sweep_max_groups(c->nc))) p *= 2;
-    S -= S % p;
-    const size_t smem = (size_t)S * slot + (size_t)S * sizeof(unsigned long long) +
-                        (size_t)sweep_max_groups(c->nc) * (ns + 1) * c->nc * sizeof(double);
-    int rc;
-    if ((rc = cuda_check(c, cudaFuncSetAttribute(k_ilu_sweeps_bulk<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                         "smem")))
-        return rc;
-    int dev = 0, nsm = 0, perSm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if ((rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_ilu_sweeps_bulk<T>, kSweepThreads, smem),
-                         "occupancy")))
-        return rc;
-    if (perSm < 1) return FP_OK;
-    *S_out = S;
-    *grid_out = std::max(1, std::min(c->hm.nElem, nsm * perSm));
-    *smem_out = smem;
-    return FP_OK;
-}
-
-template <class T>
-int launch_sweeps(fp_ctx* c, const T* F, const double* b, double* xx, unsigned epoch) {
+static int launch_register(fp_ctx* c, const T* F, const double* b, double* xx) {
     int nc = c->nc, nf = c->hm.nf, ld = c->hm.ld, nE = c->hm.nElem;
+    const size_t words = 2 * (size_t)nE * nc;
+    unsigned epoch = ++c->ilu_epoch;
+    if (epoch == 0 || c->ring_pub_ready) {  // wrapped, or words of the other kernel: clear them and start again
+        int rc = cuda_check(c, cudaMemsetAsync(c->d_ilu_pub, 0, 2 * words * sizeof(unsigned long long), c->stream), "memset");
+        if (rc) return rc;
+        epoch = c->ilu_epoch = 1;
+        c->ring_pub_ready = false;
+    }
     unsigned long long* pubF = c->d_ilu_pub;
-    unsigned long long* pubB = c->d_ilu_pub + 2 * (size_t)nE * nc;
+    unsigned long long* pubB = c->d_ilu_pub + words;
     unsigned* abortw = c->d_iluFlags;
     unsigned* status = abortw + 1;
     int polls = c->ilu_max_polls;
-    const int pi = sizeof(T) == sizeof(float) ? 1 : 0;
-    if (c->sweep_bulk_grid[pi] < 0) {
-        int S = 0, grid = 0;
-        size_t smem = 0;
-        int rc = bulk_sweep_config<T>(c, &S, &grid, &smem);
-        if (rc) return rc;
-        c->sweep_bulk_S[pi] = S;
-        c->sweep_bulk_NG[pi] = 0;  // groups per block: chosen by timing at the first application
-        c->sweep_bulk_grid[pi] = grid;
-        c->sweep_bulk_smem[pi] = smem;
-    }
-    auto launch_bulk = [&](int NG) {
-        int S = c->sweep_bulk_S[pi];
-        const int* caseOf = c->batch_mask ? c->d_case_of : nullptr;
-        const int* live = c->batch_mask ? c->d_blive : nullptr;
-        void* args[] = {&nc, &nf, &ld, &nE, &S, &NG, &c->d_swEl, &c->d_swNb, (void*)&F, (void*)&b, &xx, &pubF, &pubB,
-                        &epoch, &abortw, &status, &polls, (void*)&caseOf, (void*)&live};
-        return cudaLaunchCooperativeKernel((const void*)k_ilu_sweeps_bulk<T>, dim3(c->sweep_bulk_grid[pi]),
-                                           dim3(kSweepThreads), args, c->sweep_bulk_smem[pi], c->stream);
-    };
-    if (c->sweep_variant >= 2 && c->sweep_bulk_grid[pi] > 0) {  // a fixed group count: 2 .. 6 -> 1 .. 16
-        const int NG = 1 << (c->sweep_variant - 2);
-        if (c->sweep_bulk_S[pi] % NG != 0 || NG > sweep_max_groups(nc))
-            return set_err(c, FP_ERR_UNSUPPORTED, "ILU sweeps: group count above the slots or the block size allows");
-        return cuda_check(c, launch_bulk(NG), "ILU sweeps");
-    }
-    if (c->sweep_variant == 0 && c->sweep_bulk_grid[pi] > 0 && c->sweep_bulk_NG[pi] == 0) {
-        // autotuning: every group count NG whose slots divide evenly is timed on this application
-        // (each candidate computes the same values, so the choice never changes a result) and the
-        // fastest is kept for the context and precision
-        float best = 1e30f;
-        int bestNG = 1;
-        cudaEvent_t ev[2];
-        int rc = cuda_check(c, cudaEventCreate(&ev[0]), "event");
-        if (!rc) rc = cuda_check(c, cudaEventCreate(&ev[1]), "event");
-        if (rc) return rc;
-        for (int NG = 1; NG <= sweep_max_groups(nc) && !rc; NG *= 2) {
-            if (c->sweep_bulk_S[pi] % NG != 0) continue;
-            if (NG > 1) {  // a fresh epoch for every further candidate
-                epoch = ++c->ilu_epoch;
-                if (epoch == 0) {
-                    rc = cuda_check(c, cudaMemsetAsync(c->d_ilu_pub, 0, 4 * (size_t)nE * nc * sizeof(unsigned long long),
-                                                       c->stream), "memset");
-                    epoch = c->ilu_epoch = 1;
-                }
-            }
-            cudaEventRecord(ev[0], c->stream);
-            if (!rc) rc = cuda_check(c, launch_bulk(NG), "ILU sweeps");
-            cudaEventRecord(ev[1], c->stream);
-            float ms = 0;
-            if (!rc) rc = cuda_check(c, cudaEventSynchronize(ev[1]), "sync");
-            if (!rc) cudaEventElapsedTime(&ms, ev[0], ev[1]);
-            if (!rc && ms < best) {
-                best = ms;
-                bestNG = NG;
-            }
-        }
-        cudaEventDestroy(ev[0]);
-        cudaEventDestroy(ev[1]);
-        if (rc) return rc;
-        c->sweep_bulk_NG[pi] = bestNG;
-        return FP_OK;
-    }
-    cudaError_t e;
-    if (c->sweep_variant == 0 && c->sweep_bulk_grid[pi] > 0) {
-        e = launch_bulk(c->sweep_bulk_NG[pi]);
-    } else {
-        void* args[] = {&nc, &nf, &ld, &nE, &c->d_swEl, &c->d_swNb, (void*)&F, (void*)&b, &xx, &pubF, &pubB, &epoch,
-                        &abortw, &status, &polls};
-        e = cudaLaunchCooperativeKernel((const void*)k_ilu_sweeps<T>, dim3(c->sweep_grid), dim3(kSweepThreads), args, 0,
-                                        c->stream);
-    }
-    return cuda_check(c, e, "ILU sweeps");
+    void* args[] = {&nc, &nf, &ld, &nE, &c->d_swEl, &c->d_swNb, (void*)&F, (void*)&b, &xx, &pubF, &pubB, &epoch,
+                    &abortw, &status, &polls};
+    return cuda_check(c,
+                      cudaLaunchCooperativeKernel((const void*)k_ilu_sweeps<T>, dim3(c->sweep_grid), dim3(kSweepThreads), args, 0,
+                                                  c->stream),
+                      "ILU sweeps");
+}
+
+// Elements in flight per thread block that fp_set_ilu_sweep(ctx, 2 .. 6) may ask for: a power of
+// two up to 16 for nc <= 16, 8 for nc <= 32, else 4, and no more than a budget of whole positions
+// (all 1 + nf blocks) in shared memory, 208 KB above 32 unknowns, 100 KB below, divides into
+static bool sweep_groups_allowed(fp_ctx* c, int precision, int NG) {
+    const int nc = c->nc, most = nc <= 16 ? 16 : nc <= 32 ? 8 : 4;
+    const size_t slot = (size_t)(1 + c->hm.nf) * nc * nc * (precision == FP_PREC_FP32 ? sizeof(float) : sizeof(double));
+    const int S = (int)std::min<size_t>(32, (size_t)(nc > 32 ? 208 : 100) * 1024 / slot);
+    int p = 2;
+    while (2 * p <= std::min(S, most)) p *= 2;
+    return NG <= most && (S - S % p) % NG == 0;
 }
 
 int ilu_apply(fp_ctx* c, const double* x, double* y) {
-    const int nc = c->nc, nE = c->hm.nElem;
     if (c->ilu_prec != FP_PREC_FP32 && c->ilu_prec != FP_PREC_FP64) return set_err(c, FP_ERR_STATE, "block ILU(0): not factorised");
-    unsigned epoch = ++c->ilu_epoch;
-    if (epoch == 0) {  // wrapped: clear the published words and start again
-        int rc = cuda_check(
-            c, cudaMemsetAsync(c->d_ilu_pub, 0, 4 * (size_t)nE * nc * sizeof(unsigned long long), c->stream), "memset");
-        if (rc) return rc;
-        epoch = c->ilu_epoch = 1;
+    if (c->sweep_variant != 1 && ring_sweep_applies(c->nc)) {
+        const int NG = c->sweep_variant >= 2 ? 1 << (c->sweep_variant - 2) : 0;
+        if (NG && !sweep_groups_allowed(c, c->ilu_prec, NG))
+            return set_err(c, FP_ERR_UNSUPPORTED, "ILU sweeps: group count above the slots or the block size allows");
+        return ring_sweep(c, c->ilu_prec, x, y, NG);
     }
-    if (c->ilu_prec == FP_PREC_FP32) return launch_sweeps<float>(c, c->d_iluF32, x, y, epoch);
-    return launch_sweeps<double>(c, c->d_iluF64, x, y, epoch);
+    if (c->ilu_prec == FP_PREC_FP32) return launch_register<float>(c, c->d_iluF32, x, y);
+    return launch_register<double>(c, c->d_iluF64, x, y);
 }
 
 int ilu_check(fp_ctx* c) {
@@ -1207,6 +861,7 @@ int ilu_check(fp_ctx* c) {
         return rc;
     if (h[0] || h[1]) {
         cudaMemsetAsync(words, 0, sizeof(h), c->stream);
+        c->ring_pub_ready = false;  // what was published is unknown
         return set_err(c, FP_ERR_TIMEOUT, "block ILU(0) sweep: a dependency wait gave up");
     }
     return FP_OK;
