@@ -233,6 +233,7 @@ int ilu_factor(fp_ctx* c, int precision);                        // block ILU(0)
 int ilu_prepare_direct(fp_ctx* c, int precision, void** F);      // factor storage for blocks written in place
 int ilu_factor_direct(fp_ctx* c, int precision);                 // factorise the blocks written in place
 int ilu_apply(fp_ctx* c, const double* x, double* y);
+int ilu_rows(fp_ctx* c, void* F, bool fp32, unsigned epoch);     // fp_ilu_factor.cu
 bool ring_sweep_applies(int nc);                                 // fp_ilu_ring.cu
 int ring_sweep(fp_ctx* c, int precision, const double* b, double* x, int groups);  // groups 0: all
 int ilu_check(fp_ctx* c);                                        // FP_ERR_TIMEOUT if a sweep wait gave up

@@ -13,11 +13,10 @@
 //   * factor values in element-major storage, F[e][s][c][r] (column-major blocks):
 //     s = 0 holds inv(U_ee), s = 1 + k the block coupling e with its neighbour over face
 //     k (L or U);
-//   * rows whose lower neighbours are all finished form a level.  The factorisation is
-//     ONE persistent cooperative kernel, one 512-thread block per row in shared memory
-//     (register-tiled block products, register-resident Gauss-Jordan with implicit
-//     partial pivoting); thread blocks take the rows in level order and each row waits
-//     (bounded) only for the completion flags of its lower neighbours;
+//   * rows whose lower neighbours are all finished form a level.  The factorisation is ONE
+//     persistent cooperative kernel (fp_ilu_factor.cu), one thread block per row in shared
+//     memory; thread blocks take the rows in level order and each row waits (bounded) only for
+//     the completion flags of its lower neighbours;
 //   * an application (forward L sweep, backward U sweep) is ONE persistent cooperative
 //     kernel: thread blocks take the elements in level order, and each element waits
 //     (bounded) only for the values of the neighbours it multiplies, so levels overlap and no
@@ -29,8 +28,6 @@
 //     mixed-precision GMRES, where the blocks are either gathered from the assembled
 //     operator (rounded) or written straight into the FP32 factor storage by the exact
 //     Jacobian kernel (no FP64 copy of the blocks exists then), and factorised in place.
-#include <cuda_pipeline.h>
-
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -41,7 +38,6 @@ namespace fp {
 
 namespace {
 
-constexpr int kFactorThreads = 512;
 constexpr int kSweepThreads = 512;
 constexpr int kMaxNc = 64;   // unknowns per element
 constexpr int kMaxF = 4;     // faces per element
@@ -92,240 +88,9 @@ __global__ void __launch_bounds__(256) k_ilu_gather(int nElem, int ld, int nc, i
     }
 }
 
-// C (-)= X * Y for nc x nc column-major blocks in shared memory (nc <= 64): thread t
-// computes the 4 x 4 tile (rows 4 (t % 16) .., columns 4 (t / 16) ..), so each value read
-// from shared memory feeds four multiply-adds (the products are bound by shared-memory
-// wavefronts, not by the FP64 pipe).
-template <class T>
-__device__ __forceinline__ void block_mul(int nc, const T* X, const T* Y, T* C, bool subtract) {
-    const int t = threadIdx.x;
-    const int r0 = 4 * (t & 15), c0 = 4 * (t >> 4);
-    if (r0 >= nc || c0 >= nc) return;
-    T acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-    for (int m = 0; m < nc; m++) {
-        T x[4], y[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) x[a] = r0 + a < nc ? X[m * nc + r0 + a] : T(0);
-#pragma unroll
-        for (int b = 0; b < 4; b++) y[b] = c0 + b < nc ? Y[(c0 + b) * nc + m] : T(0);
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] += x[a] * y[b];
-    }
-#pragma unroll
-    for (int b = 0; b < 4; b++)
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-            if (r0 + a < nc && c0 + b < nc) {
-                T* cp = C + (c0 + b) * nc + r0 + a;
-                if (subtract)
-                    *cp -= acc[a][b];
-                else
-                    *cp = acc[a][b];
-            }
-}
-
-// Inverse of the nc x nc column-major block A (shared memory) into out (column-major,
-// global memory) by Gauss-Jordan on [A | I] with implicit partial pivoting and unscaled
-// pivot rows.  Thread (row r = t % 64, column group cg = t / 64) keeps a_r,c for
-// c = cg + 8 (k + k0) (k < 16) in registers, where k0 = p / 8 counts the register shifts
-// made so far (every 8 steps the array moves down by one, dropping a left-half column
-// that is no longer read, so the pivot column always sits in a[0] and no register is
-// indexed at run time).  Step p: the owners of column p publish it, every warp finds the
-// pivot row br (the unused row with the largest |a_rp|, compared in single precision)
-// itself, the owners of row br publish it, and each
-// thread updates a_rc -= (a_rp / a_br,p) a_br,c for its c > p.  The published column and
-// row are double-buffered, so two barriers per step suffice; columns <= p of the left
-// half are left stale.  At the end row stepOfRow^-1(p) holds d_p e_p on the left and d_p
-// times row p of inv(A) on the right, d_p its pivot.  512 threads.  A singular block sets
-// FP_DEV_SINGULAR in *status and returns false.  T is the arithmetic type (the factors').
-template <class T>
-__device__ __forceinline__ bool gj_inverse(int nc, const T* A, T* colbuf, T* rowbuf, int* stepOfRow, T* pivOfRow, T* out,
-                                           unsigned* status) {
-    __shared__ T pivInv[2];
-    const int t = threadIdx.x, n2 = 2 * nc;
-    const int r = t & 63, cg = t >> 6, lane = t & 31;
-    T a[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) {
-        const int c = cg + 8 * k;
-        a[k] = T(0);
-        if (r < nc && c < nc) a[k] = A[c * nc + r];
-        if (r < nc && c >= nc && c < n2) a[k] = (c - nc == r) ? T(1) : T(0);
-    }
-    unsigned long long usedMask = 0ull;
-    bool singular = false;
-    int k0 = 0;
-    for (int p = 0; p < nc; p++) {
-        T* colp = colbuf + (p & 1) * 64;
-        T* rowp = rowbuf + (p & 1) * 128;
-        if (cg == (p & 7) && r < nc) colp[r] = a[0];
-        __syncthreads();
-        // pivot key: the bits of (float)|a_rp| (ordered like unsigned integers for
-        // non-negative floats) with the low 6 bits replaced by 63 - r, reduced by one
-        // warp-wide unsigned max; ties in the leading 18 bits go to the lowest row
-        unsigned key = 0u;
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int rr = lane + 32 * k;
-            if (rr < nc && !((usedMask >> rr) & 1ull)) {
-                const T v = fabs(colp[rr]);
-                unsigned kb = __float_as_uint((float)v) & ~63u;
-                if (kb == 0u && v > T(0)) kb = 64u;  // below float range: still a candidate
-                if (!isfinite(v)) kb = 0xffffffc0u;
-                key = max(key, kb | (unsigned)(63 - rr));
-            }
-        }
-        key = __reduce_max_sync(0xffffffffu, key);
-        const int br = 63 - (int)(key & 63u);
-        const T bv = br < nc ? fabs(colp[br]) : T(0);
-        if (key < 64u || !(bv > T(0)) || !isfinite(bv)) {  // the same decision in every warp
-            singular = true;
-            break;
-        }
-        usedMask |= 1ull << br;
-        if (r == br) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int c = cg + 8 * (k + k0);
-                if (c < n2) rowp[c] = a[k];
-            }
-        }
-        if (t == 0) {
-            stepOfRow[br] = p;
-            pivOfRow[br] = colp[br];
-            pivInv[p & 1] = T(1) / colp[br];
-        }
-        __syncthreads();
-        if (r < nc && r != br) {
-            const T m = colp[r] * pivInv[p & 1];
-#pragma unroll
-            for (int k = 0; k < 16; k++) {
-                const int c = cg + 8 * (k + k0);
-                if (c > p && c < n2) a[k] -= m * rowp[c];
-            }
-        }
-        if ((p & 7) == 7) {
-#pragma unroll
-            for (int k = 0; k < 15; k++) a[k] = a[k + 1];
-            a[15] = T(0);
-            k0++;
-        }
-    }
-    if (singular) {
-        if (t == 0) atomicOr(status, (unsigned)FP_DEV_SINGULAR);
-        return false;
-    }
-    __syncthreads();
-    // row r holds d times row stepOfRow[r] of the inverse in its right half
-    if (r < nc) {
-        const int pr = stepOfRow[r];
-        const T d = pivOfRow[r];
-#pragma unroll
-        for (int k = 0; k < 16; k++) {
-            const int c = cg + 8 * (k + k0);
-            if (c >= nc && c < n2) out[(c - nc) * nc + pr] = a[k] / d;
-        }
-    }
-    return true;
-}
-
-// completion flags of the factorisation rows: release by the producer, acquire by the consumers
-__device__ __forceinline__ unsigned flag_load(const unsigned* f) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-    return v;
-}
-__device__ __forceinline__ void flag_store(unsigned* f, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(f), "r"(v) : "memory");
-}
-
 constexpr int kSpinPolls = 1 << 12;  // polled back to back first (a dependency is usually microseconds away)
 // then with 64 ns sleeps up to the context's limit (default 2^19 polls: a wait gives up well
 // within a second; a context may lower it, down to 0, so that tests can make a wait run out)
-
-// Bounded wait until *f == epoch.  A wait that runs out sets FP_DEV_TIMEOUT and the abort
-// word, which ends every other wait of the launch at once; the results are then garbage
-// and the host reports the timeout.
-__device__ __forceinline__ void flag_wait(const unsigned* f, unsigned epoch, unsigned* abortw, unsigned* status,
-                                          int maxPolls) {
-    for (int it = 0; it < maxPolls; it++) {
-        if (flag_load(f) == epoch) return;
-        if ((it & 31) == 31 && *(volatile unsigned*)abortw) return;
-        if (it >= kSpinPolls) __nanosleep(64);
-    }
-    atomicOr(status, (unsigned)FP_DEV_TIMEOUT);
-    atomicExch(abortw, 1u);
-}
-
-// The factorisation in one persistent launch: thread block g takes the rows g, g +
-// gridDim.x, ... in forward-level order, one 512-thread block per row in shared memory.
-// A row's own blocks are requested first (only the row itself changes them); then it
-// waits (bounded) for the completion flags of its lower neighbours, whose finished
-// blocks it reads, so consecutive levels overlap.  Every dependency lies in an earlier
-// level, every block walks its rows in level order and all blocks are co-resident
-// (cooperative launch), so each wait ends.  A singular diagonal block sets
-// FP_DEV_SINGULAR and still completes its row, so no dependent waits for it.  T: the
-// factors' type, in which the factorisation also computes.
-template <class T>
-__global__ void __launch_bounds__(kFactorThreads)
-    k_ilu_factor(int nc, int nf, int nE, const int* __restrict__ lvl, const int4* __restrict__ nbLow,
-                 const int* __restrict__ opPtr, const int4* __restrict__ ops, T* F, unsigned* done, unsigned epoch,
-                 unsigned* abortw, unsigned* status, int maxPolls, unsigned* sing) {
-    extern __shared__ __align__(16) unsigned char ilu_smem[];
-    T* sm = reinterpret_cast<T*>(ilu_smem);
-    const int nc2 = nc * nc, ns = 1 + nf;
-    const int t = threadIdx.x;
-    T* R = sm;             // [ns][nc2] the row's blocks
-    T* Lb = R + ns * nc2;  // current L block
-    T* Yb = Lb + nc2;      // staging of row k's block
-    __shared__ T colbuf[2 * kMaxNc], rowbuf[4 * kMaxNc], pivOfRow[kMaxNc];
-    __shared__ int stepOfRow[kMaxNc];
-    for (int q0 = blockIdx.x; q0 < nE; q0 += gridDim.x) {
-        const int i = lvl[q0];
-        T* Fi = F + (size_t)i * ns * nc2;
-        // global -> shared copies as asynchronous element copies: all of a thread's copies
-        // are in flight together instead of one DRAM round trip per loop iteration
-        for (int q = t; q < ns * nc2; q += blockDim.x) __pipeline_memcpy_async(R + q, Fi + q, sizeof(T));
-        __pipeline_commit();
-        if (t < nf) {
-            const int4 nb = nbLow[i];
-            const int k = t == 0 ? nb.x : t == 1 ? nb.y : t == 2 ? nb.z : nb.w;
-            if (k >= 0) flag_wait(done + k, epoch, abortw, status, maxPolls);
-        }
-        for (int q = opPtr[i]; q < opPtr[i + 1]; q++) {
-            const int4 op = ops[q];
-            // block of row k: inv(U_kk) for an L step, U_kj for an update
-            const T* Y = F + ((size_t)op.z * ns + (op.x == 0 ? 0 : 1 + op.w)) * nc2;
-            __syncthreads();
-            for (int u = t; u < nc2; u += blockDim.x) __pipeline_memcpy_async(Yb + u, Y + u, sizeof(T));
-            __pipeline_commit();
-            __pipeline_wait_prior(0);
-            __syncthreads();
-            if (op.x == 0) {
-                // L = A_ik * inv(U_kk)
-                block_mul(nc, R + (size_t)(1 + op.y) * nc2, Yb, Lb, false);
-                __syncthreads();
-                for (int u = t; u < nc2; u += blockDim.x) R[(size_t)(1 + op.y) * nc2 + u] = Lb[u];
-            } else {
-                // A_ij -= L * U_kj
-                block_mul(nc, Lb, Yb, R + (size_t)op.y * nc2, true);
-            }
-        }
-        __pipeline_wait_prior(0);
-        __syncthreads();
-        // inverse of the updated diagonal block
-        if (!gj_inverse(nc, R, colbuf, rowbuf, stepOfRow, pivOfRow, Fi, status) && t == 0) sing[i] = 1u;  // the row's mark
-        for (int u = nc2 + t; u < ns * nc2; u += blockDim.x) Fi[u] = R[u];
-        __syncthreads();  // the row is written (and the shared buffers are free again)
-        if (t == 0) flag_store(done + i, epoch);
-    }
-}
 
 // Lanes per row in the sweeps: the largest power of two G <= 32 with G nc <= 512, so a
 // row's G lanes are adjacent in one warp and meet by shuffles.
@@ -677,40 +442,17 @@ int ilu_check_sizes(fp_ctx* c) {
 template <class T>
 int ilu_factor_run(fp_ctx* c, T* F) {
     int rc;
-    const int nc = c->nc, nf = c->hm.nf, nE = c->hm.nElem;
-    const size_t nc2 = (size_t)nc * nc;
-    const size_t smem = ((size_t)(1 + nf) * nc2 + 2 * nc2) * sizeof(T);
+    const int nE = c->hm.nElem;
     if ((rc = cuda_check(c, cudaMemsetAsync(c->d_status, 0, sizeof(unsigned), c->stream), "memset"))) return rc;
-    if (smem > 48 * 1024 &&
-        (rc = cuda_check(c, cudaFuncSetAttribute(k_ilu_factor<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                         "smem")))
-        return rc;
-    // persistent factorisation grid: every block co-resident (cooperative launch)
-    int dev = 0, nsm = 0, perSm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if ((rc = cuda_check(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_ilu_factor<T>, kFactorThreads, smem),
-                         "occupancy")))
-        return rc;
-    if (perSm < 1) return set_err(c, FP_ERR_UNSUPPORTED, "block ILU(0): factorisation block does not fit an SM");
     unsigned* abortw = c->d_iluFlags;
-    unsigned* done = c->d_iluFlags + 2;
     unsigned epoch = ++c->ilu_fepoch;
     if (epoch == 0) {  // wrapped: clear the row flags and start again
-        if ((rc = cuda_check(c, cudaMemsetAsync(done, 0, (size_t)nE * sizeof(unsigned), c->stream), "memset"))) return rc;
+        if ((rc = cuda_check(c, cudaMemsetAsync(c->d_iluFlags + 2, 0, (size_t)nE * sizeof(unsigned), c->stream), "memset")))
+            return rc;
         epoch = c->ilu_fepoch = 1;
     }
-    int nEl = nE, ncl = nc, nfl = nf, polls = c->ilu_max_polls;
-    unsigned* status = c->d_status;
-    unsigned* sing = c->d_ilu_sing;
-    if ((rc = cuda_check(c, cudaMemsetAsync(sing, 0, (size_t)nE * sizeof(unsigned), c->stream), "memset"))) return rc;
-    void* args[] = {&ncl, &nfl, &nEl, &c->d_lvlF, &c->d_nbLow, &c->d_opPtr, &c->d_ops, &F, &done, &epoch, &abortw,
-                    &status, &polls, &sing};
-    const int grid = std::max(1, std::min(nE, nsm * perSm));
-    if ((rc = cuda_check(c,
-                         cudaLaunchCooperativeKernel((const void*)k_ilu_factor<T>, dim3(grid), dim3(kFactorThreads), args,
-                                                     smem, c->stream),
-                         "ILU factor")))
+    if ((rc = cuda_check(c, cudaMemsetAsync(c->d_ilu_sing, 0, (size_t)nE * sizeof(unsigned), c->stream), "memset")) ||
+        (rc = ilu_rows(c, F, sizeof(T) == sizeof(float), epoch)))
         return rc;
     unsigned st = 0;
     if ((rc = cuda_check(c, cudaMemcpyAsync(&st, c->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream), "copy")) ||
