@@ -132,23 +132,84 @@ struct Element {
     static constexpr int NB = TB::NB, NQV = TB::NQV, NQF = TB::NQF, NF = TB::NF, NV = TB::NV, NVF = TB::NVF, NP = TB::NP;
     static constexpr int NE = Mdl::NE, NC = NE * NB;
 
+    // Whether a face's integrand reads the gradients of the traces: always for viscous models,
+    // otherwise only through the artificial viscosity of an interior face (a coefficient of exactly
+    // zero adds nothing, so the values without the gradients are the same bits).
+    static __device__ __forceinline__ bool needs_gradients(const DevMesh& M, bool interior, double eps_e, double eps_nb) {
+        return Mdl::kViscous || (interior && 0.5 * (eps_e + eps_nb) + M.dampConst != 0.0);
+    }
+
     // One face quadrature point of DGpure.residuumWall (DGpure.java:204-353) seen from element
     // e (owner side): C = -(fn - vn Wale) + avFlux + fvn and Jmp = WL - WR (after the flux
     // calls have limited the densities in place, as Java's arrays are), so that the element's
     // integrand is C - c_IP Jmp (interior faces and IP walls) and the neighbour's -C + c_IP' Jmp.
     // w: the owner's coefficients, a register array or an accessor reading them from memory
-    template <class T, class OwnL, class NbL>
+    // GRAD: with the gradients of the traces (needs_gradients)
+    template <bool GRAD, class T, class OwnL, class NbL>
     static __device__ __forceinline__ void face_point(const DevMesh& M, int e, int k, int p, int TT, const double* n,
                                                       double dL, const double* Jinv, const double* JinvR, int kr_face,
                                                       int pm, double eps_e, double eps_nb, const OwnL& w, const NbL& nbl,
                                                       T* C, T* Jmp) {
+        const double* tab = M.tab;
+        const double* phiL = tab + TB::o_phiL + (k * NQF + p) * NB;
+        const double* dphiL = tab + TB::o_dphiL + (k * NQF + p) * NB * DIM;
+        // traces (DGpure.java:239-264)
+        constexpr int NG = GRAD ? DIM * NE : 1;
+        T WL[NE], WR[NE], dWL[NG], dWR[NG];
+        trace<GRAD>(phiL, dphiL, Jinv, [&](int c) { return w[c]; }, WL, dWL);
+        if (TT > -1) {
+            const double* phiR = tab + TB::o_phiR + ((kr_face * NP + pm) * NQF + p) * NB;
+            const double* dphiR = tab + TB::o_dphiR + ((kr_face * NP + pm) * NQF + p) * NB * DIM;
+            trace<GRAD>(phiR, dphiR, JinvR, [&](int c) { return nbl(c, TT); }, WR, dWR);
+        }
+        point_flux<GRAD>(M, e, k, p, TT, n, dL, eps_e, eps_nb, WL, WR, dWL, dWR, C, Jmp);
+    }
+
+    // value and (GRAD) physical gradient of the coefficients coef(c) at one point
+    template <bool GRAD, class T, class Coef>
+    static __device__ __forceinline__ void trace(const double* phi, const double* dphi, const double* Ji, const Coef& coef,
+                                                 T* W, T* dW) {
+        constexpr int NG = GRAD ? DIM * NE : 1;
+        T g[NG];
+#pragma unroll
+        for (int m = 0; m < NE; m++) {
+            W[m] = 0.0;
+            if constexpr (GRAD) {
+#pragma unroll
+                for (int d = 0; d < DIM; d++) g[d * NE + m] = 0.0;
+            }
+#pragma unroll
+            for (int j = 0; j < NB; j++) {
+                const T c = coef(m * NB + j);
+                W[m] += c * ldg(phi + j);
+                if constexpr (GRAD) {
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) g[d * NE + m] += c * ldg(dphi + j * DIM + d);
+                }
+            }
+        }
+        if constexpr (GRAD) {
+#pragma unroll
+            for (int m = 0; m < NE; m++)
+#pragma unroll
+                for (int d = 0; d < DIM; d++) {
+                    T s = 0.0;
+#pragma unroll
+                    for (int q = 0; q < DIM; q++) s += Ji[q * DIM + d] * g[q * NE + m];
+                    dW[d * NE + m] = s;
+                }
+        }
+    }
+
+    // the integrand of face_point from the traces WL and, on interior faces, WR (dWL, dWR with GRAD)
+    template <bool GRAD, class T>
+    static __device__ __forceinline__ void point_flux(const DevMesh& M, int e, int k, int p, int TT, const double* n, double dL,
+                                                      double eps_e, double eps_nb, T* WL, T* WR, T* dWL, T* dWR, T* C, T* Jmp) {
         const int ld = M.ld;
         const double* geo = M.geo;
         const double* tab = M.tab;
         const fp_model_params& P = M.P;
         const bool interior = TT > -1;
-        const double* phiL = tab + TB::o_phiL + (k * NQF + p) * NB;
-        const double* dphiL = tab + TB::o_dphiL + (k * NQF + p) * NB * DIM;
         // mesh velocity and position at the face point (Element.java:299-332)
         double u[DIM];
 #pragma unroll
@@ -173,64 +234,13 @@ struct Element {
                 X[i] = s + ldg(geo + (size_t)(GL::X0 + i) * ld + e);
             }
         }
-        // traces (DGpure.java:239-264)
-        T WL[NE], WR[NE], dWL[DIM * NE], dWR[DIM * NE];
-        {
-            T g[DIM * NE];
-#pragma unroll
-            for (int m = 0; m < NE; m++) {
-                WL[m] = 0.0;
-#pragma unroll
-                for (int d = 0; d < DIM; d++) g[d * NE + m] = 0.0;
-#pragma unroll
-                for (int j = 0; j < NB; j++) {
-                    const T& c = w[m * NB + j];
-                    WL[m] += c * ldg(phiL + j);
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) g[d * NE + m] += c * ldg(dphiL + j * DIM + d);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < NE; m++)
-#pragma unroll
-                for (int d = 0; d < DIM; d++) {
-                    T s = 0.0;
-#pragma unroll
-                    for (int q = 0; q < DIM; q++) s += Jinv[q * DIM + d] * g[q * NE + m];
-                    dWL[d * NE + m] = s;
-                }
-        }
-        if (interior) {
-            const double* phiR = tab + TB::o_phiR + ((kr_face * NP + pm) * NQF + p) * NB;
-            const double* dphiR = tab + TB::o_dphiR + ((kr_face * NP + pm) * NQF + p) * NB * DIM;
-            T g[DIM * NE];
-#pragma unroll
-            for (int m = 0; m < NE; m++) {
-                WR[m] = 0.0;
-#pragma unroll
-                for (int d = 0; d < DIM; d++) g[d * NE + m] = 0.0;
-#pragma unroll
-                for (int j = 0; j < NB; j++) {
-                    const T c = nbl(m * NB + j, TT);
-                    WR[m] += c * ldg(phiR + j);
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) g[d * NE + m] += c * ldg(dphiR + j * DIM + d);
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < NE; m++)
-#pragma unroll
-                for (int d = 0; d < DIM; d++) {
-                    T s = 0.0;
-#pragma unroll
-                    for (int q = 0; q < DIM; q++) s += JinvR[q * DIM + d] * g[q * NE + m];
-                    dWR[d * NE + m] = s;
-                }
-        } else {
+        if (!interior) {
             // the outlet pressure of the element's case in a batch of cases, else the model's
             Mdl::boundaryValue(WL, n, TT, u, X, WR, P, M.case_pout ? ldg(M.case_pout + M.case_of[e]) : P.p_out);
+            if constexpr (GRAD) {
 #pragma unroll
-            for (int i = 0; i < DIM * NE; i++) dWR[i] = dWL[i];
+                for (int i = 0; i < DIM * NE; i++) dWR[i] = dWL[i];
+            }
         }
         // inviscid flux (DGpure.java:266-281)
         double vn = 0;
@@ -254,7 +264,7 @@ struct Element {
         const double idL = 1.0 / dL;
         // DDG viscous flux (DGpure.java:283-303)
         T fvn[NE];
-        if (Mdl::kViscous) {
+        if constexpr (Mdl::kViscous) {
             T Wc[NE], dWc[NE * DIM];
 #pragma unroll
             for (int m = 0; m < NE; m++) {
@@ -276,14 +286,16 @@ struct Element {
 #pragma unroll
         for (int m = 0; m < NE; m++) {
             T g = -(fn[m] - vn * Wale[m]);
-            if (interior) {
-                T dWsum = 0.0;
+            if constexpr (GRAD) {
+                if (interior) {
+                    T dWsum = 0.0;
 #pragma unroll
-                for (int d = 0; d < DIM; d++) dWsum += (dWL[NE * d + m] + dWR[NE * d + m]) / 2.0 * n[d];
-                const double epsFace = 0.5 * (eps_e + eps_nb) + M.dampConst;
-                g += epsFace * (dWsum + M.beta0 * (WR[m] - WL[m]) * idL);
+                    for (int d = 0; d < DIM; d++) dWsum += (dWL[NE * d + m] + dWR[NE * d + m]) / 2.0 * n[d];
+                    const double epsFace = 0.5 * (eps_e + eps_nb) + M.dampConst;
+                    g += epsFace * (dWsum + M.beta0 * (WR[m] - WL[m]) * idL);
+                }
             }
-            if (Mdl::kViscous) g += fvn[m];
+            if constexpr (Mdl::kViscous) g += fvn[m];
             C[m] = g;
             Jmp[m] = WL[m] - WR[m];
         }
@@ -329,11 +341,19 @@ struct Element {
                 eps_nb = ldg(M.eps + TT);
             }
             const bool ip = Mdl::kViscous && (interior || Mdl::isIPFace(TT));
+            const bool grads = needs_gradients(M, interior, eps_e, eps_nb);
             if (KR::enabled && interior) kr.template begin<T>(k);
 #pragma unroll 1
             for (int p = 0; p < NQF; p++) {
                 T C[NE], Jm[NE];
-                face_point(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+                if constexpr (Mdl::kViscous) {
+                    face_point<true>(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+                } else {
+                    if (grads)
+                        face_point<true>(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+                    else
+                        face_point<false>(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+                }
                 const double jw = Jac * ldg(M.tab + TB::o_wf + p);
                 const double* phiL = M.tab + TB::o_phiL + (k * NQF + p) * NB;
 #pragma unroll
@@ -428,30 +448,12 @@ struct Element {
                 }
             }
             T WI[NE], dWI[DIM * NE];
-            {
-                T g[DIM * NE];
+            if (Mdl::kViscous || Mdl::kSource || avc != 0.0) {
+                trace<true>(phi, dphi, Jinv, [&](int c) { return w[c]; }, WI, dWI);
+            } else {  // nothing reads the gradient: its coefficient is exactly zero
+                trace<false>(phi, dphi, Jinv, [&](int c) { return w[c]; }, WI, dWI);
 #pragma unroll
-                for (int m = 0; m < NE; m++) {
-                    WI[m] = 0.0;
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) g[d * NE + m] = 0.0;
-#pragma unroll
-                    for (int j = 0; j < NB; j++) {
-                        const T& c = w[m * NB + j];
-                        WI[m] += c * ldg(phi + j);
-#pragma unroll
-                        for (int d = 0; d < DIM; d++) g[d * NE + m] += c * ldg(dphi + j * DIM + d);
-                    }
-                }
-#pragma unroll
-                for (int m = 0; m < NE; m++)
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) {
-                        T s = 0.0;
-#pragma unroll
-                        for (int qq = 0; qq < DIM; qq++) s += Jinv[qq * DIM + d] * g[qq * NE + m];
-                        dWI[d * NE + m] = s;
-                    }
+                for (int i = 0; i < DIM * NE; i++) dWI[i] = 0.0;
             }
             const double jw = jac * weight;
             // G[d][m]: coefficient of d(phi_j)/dx_d, then mapped to the reference gradient
