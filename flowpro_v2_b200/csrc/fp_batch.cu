@@ -25,10 +25,20 @@ namespace fp {
 
 namespace {
 
-constexpr int kChunk = 2048;  // elements per chunk of the segmented reductions
 constexpr int kRT = 256;
 
-inline unsigned vgrid_of(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16); }
+// Elements per chunk of the segmented reductions, a power of two: small enough that the chunks of a
+// few small cases still fill the GPU (16,600 triangles of 40 unknowns: 2,048 elements a chunk were 10
+// thread blocks and 267 us a dot product pass, 64 are 260 and 16 us), large enough that the partial
+// sums of many cases stay few.
+inline int chunk_elements(int nElem) {
+    int n = 64;
+    while (n < 2048 && nElem / n > 8 * 148) n *= 2;
+    return n;
+}
+
+// grid of the element-parallel vector kernels: element blocks x components
+inline dim3 vgrid_of(size_t n, int K) { return dim3((unsigned)((n + 255) / 256), (unsigned)K); }
 
 constexpr int kKB = 8;  // Krylov vectors per block of the chunk dot products
 
@@ -47,9 +57,13 @@ __global__ void __launch_bounds__(kRT) k_chunk_dots(int nchunks, const int* __re
     double s[kKB];
 #pragma unroll
     for (int k = 0; k < kKB; k++) s[k] = 0.0;
-    for (int q = 0; q < K; q++) {
+    // threads over tiles of up to kRT elements, the rest of them over the components
+    int tile = 32;
+    while (tile < kRT && tile < n) tile *= 2;
+    const int el = threadIdx.x & (tile - 1), qs = kRT / tile;
+    for (int q = threadIdx.x / tile; q < K; q += qs) {
         const size_t base = (size_t)q * ld + e0;
-        for (int e = threadIdx.x; e < n; e += kRT) {
+        for (int e = el; e < n; e += tile) {
             const double av = a[base + e];
             if (!V) {
                 s[0] += av * av;
@@ -108,68 +122,66 @@ __global__ void __launch_bounds__(kRT) k_chunk_min(int nchunks, const int* __res
     if (threadIdx.x == 0) part[ch] = sh[0];
 }
 
-// out[k][case] = the case's chunk partials combined in chunk order (sum, or min when mn)
+// out[k][case] = the case's chunk partials combined (sum, or min when mn), a warp each, in a fixed order
 __global__ void k_case_combine(int ncases, const int* __restrict__ cptr, int nchunks, int K, const double* __restrict__ part,
                                double* __restrict__ out, int mn) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (t >= K * ncases) return;
     const int k = t / ncases, cs = t - k * ncases;
     double s = mn ? 1.0e300 : 0.0;
-    for (int ch = cptr[cs]; ch < cptr[cs + 1]; ch++) s = mn ? fmin(s, part[(size_t)k * nchunks + ch]) : s + part[(size_t)k * nchunks + ch];
-    out[(size_t)k * ncases + cs] = s;
+    for (int ch = cptr[cs] + lane; ch < cptr[cs + 1]; ch += 32)
+        s = mn ? fmin(s, part[(size_t)k * nchunks + ch]) : s + part[(size_t)k * nchunks + ch];
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_down_sync(0xffffffffu, s, o);
+        s = mn ? fmin(s, v) : s + v;
+    }
+    if (lane == 0) out[(size_t)k * ncases + cs] = s;
 }
+inline unsigned combine_grid(int n) { return (unsigned)((n + 3) / 4); }  // 128 threads: four (vector, case) pairs
 
-// Element-parallel vector kernels over the merged mesh: thread e handles the K components of
-// element e, reads its case once, and skips the element when the case's live flag is 0 (live ==
-// nullptr: every case), leaving its values untouched.
+// Element-parallel vector kernels over the merged mesh: thread (e, q) handles component q = blockIdx.y
+// of element e and skips it when the case's live flag is 0 (live == nullptr: every case), leaving its
+// value untouched.
 
 // w[q ld + e] += sgn * sum_{k < kc(case)} h[k][case] V_k[q ld + e] (kcs: per-case counts,
 // nullptr: kc for every case)
-__global__ void k_case_maxpy(int nElem, int ld, int K, int kc, int ncases, const int* __restrict__ case_of,
+__global__ void k_case_maxpy(int nElem, int ld, int kc, int ncases, const int* __restrict__ case_of,
                              const int* __restrict__ live, const int* __restrict__ kcs, double sgn, double* __restrict__ w,
                              const double* __restrict__ V, size_t stride, const double* __restrict__ h) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nElem; e += gridDim.x * blockDim.x) {
-        const int cs = case_of[e];
-        if (live && !live[cs]) continue;
-        const int kn = kcs ? kcs[cs] : kc;
-        for (int q = 0; q < K; q++) {
-            const size_t i = (size_t)q * ld + e;
-            double s = 0;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nElem) return;
+    const int cs = case_of[e];
+    if (live && !live[cs]) return;
+    const int kn = kcs ? kcs[cs] : kc;
+    const size_t i = (size_t)blockIdx.y * ld + e;
+    double s = 0;
 #pragma unroll 4
-            for (int k = 0; k < kn; k++) s += h[(size_t)k * ncases + cs] * V[(size_t)k * stride + i];
-            w[i] += sgn * s;
-        }
-    }
+    for (int k = 0; k < kn; k++) s += h[(size_t)k * ncases + cs] * V[(size_t)k * stride + i];
+    w[i] += sgn * s;
 }
 
 // y = x / sqrt(nrm2[case]) (0 for a zero norm)
-__global__ void k_case_normalise(int nElem, int ld, int K, const int* __restrict__ case_of, const int* __restrict__ live,
+__global__ void k_case_normalise(int nElem, int ld, const int* __restrict__ case_of, const int* __restrict__ live,
                                  const double* __restrict__ nrm2, const double* __restrict__ x, double* __restrict__ y) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nElem; e += gridDim.x * blockDim.x) {
-        const int cs = case_of[e];
-        if (live && !live[cs]) continue;
-        const double s = nrm2[cs];
-        const double r = s > 0 ? sqrt(s) : 0.0;
-        for (int q = 0; q < K; q++) {
-            const size_t i = (size_t)q * ld + e;
-            y[i] = s > 0 ? x[i] / r : 0.0;
-        }
-    }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nElem) return;
+    const int cs = case_of[e];
+    if (live && !live[cs]) return;
+    const double s = nrm2[cs];
+    const size_t i = (size_t)blockIdx.y * ld + e;
+    y[i] = s > 0 ? x[i] / sqrt(s) : 0.0;
 }
 
 // cases with mask[case] != 0: mode 0 y = x, mode 1 y += x
-__global__ void k_case_masked(int nElem, int ld, int K, const int* __restrict__ case_of, const int* __restrict__ mask, int mode,
+__global__ void k_case_masked(int nElem, int ld, const int* __restrict__ case_of, const int* __restrict__ mask, int mode,
                               const double* __restrict__ x, double* __restrict__ y) {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nElem; e += gridDim.x * blockDim.x) {
-        if (!mask[case_of[e]]) continue;
-        for (int q = 0; q < K; q++) {
-            const size_t i = (size_t)q * ld + e;
-            if (mode == 0)
-                y[i] = x[i];
-            else
-                y[i] += x[i];
-        }
-    }
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nElem || !mask[case_of[e]]) return;
+    const size_t i = (size_t)blockIdx.y * ld + e;
+    if (mode == 0)
+        y[i] = x[i];
+    else
+        y[i] += x[i];
 }
 
 __global__ void k_bminus_all(size_t n, double* __restrict__ y, const double* __restrict__ b) {
@@ -224,12 +236,13 @@ struct Batch {
 int batch_prepare(fp_ctx* c, int kmax) {
     const int n = c->n_cases;
     if (c->batch_ready && c->batch_kmax >= kmax) return FP_OK;
+    const int chunk = chunk_elements(c->hm.nElem);
     std::vector<int> e0, e1, cptr(n + 1, 0);
     for (int cs = 0; cs < n; cs++) {
         cptr[cs] = (int)e0.size();
-        for (int a = c->case_e0[cs]; a < c->case_e0[cs + 1]; a += kChunk) {
+        for (int a = c->case_e0[cs]; a < c->case_e0[cs + 1]; a += chunk) {
             e0.push_back(a);
-            e1.push_back(std::min(a + kChunk, c->case_e0[cs + 1]));
+            e1.push_back(std::min(a + chunk, c->case_e0[cs + 1]));
         }
     }
     cptr[n] = (int)e0.size();
@@ -254,7 +267,7 @@ int batch_prepare(fp_ctx* c, int kmax) {
 int case_sums(fp_ctx* c, const double* in, int K, std::vector<double>& host) {
     const int n = c->n_cases, nch = c->batch_nch;
     k_chunk_sums<<<dim3(nch, K), kRT, 0, c->stream>>>(nch, c->d_bch0, c->d_bch1, c->hm.ld, in, c->d_bpart);
-    k_case_combine<<<(K * n + 127) / 128, 128, 0, c->stream>>>(n, c->d_bcptr, nch, K, c->d_bpart, c->d_bcase, 0);
+    k_case_combine<<<combine_grid(K * n), 128, 0, c->stream>>>(n, c->d_bcptr, nch, K, c->d_bpart, c->d_bcase, 0);
     host.resize((size_t)K * n);
     int rc = cuda_check(c, cudaMemcpyAsync(host.data(), c->d_bcase, host.size() * sizeof(double), cudaMemcpyDeviceToHost,
                                            c->stream), "copy");
@@ -270,7 +283,7 @@ void case_dots(fp_ctx* c, const double* a, const double* V, int kc, double* out)
     const int ky = V ? (kc + kKB - 1) / kKB : 1;
     k_chunk_dots<<<dim3(nch, ky), kRT, 0, c->stream>>>(nch, c->d_bch0, c->d_bch1, c->d_case_of, live, c->nc, c->hm.ld, kc, a,
                                                         V, c->nvec, c->d_bpart);
-    k_case_combine<<<(kc * n + 127) / 128, 128, 0, c->stream>>>(n, c->d_bcptr, nch, kc, c->d_bpart, out, 0);
+    k_case_combine<<<combine_grid(kc * n), 128, 0, c->stream>>>(n, c->d_bcptr, nch, kc, c->d_bpart, out, 0);
 }
 
 int fetch_dev(fp_ctx* c, const double* d, size_t n, double* h) {
@@ -288,9 +301,9 @@ int batch_reset(fp_ctx* c, const std::vector<int>& mark) {
     if (!any) return FP_OK;
     int rc = upload(c, c->d_bmask, mark.data(), mark.size());
     if (rc) return rc;
-    const unsigned G = vgrid_of(c->hm.nElem);
+    const dim3 G = vgrid_of(c->hm.nElem, c->nc);
     for (double* d : {c->d_W, c->d_Wo, c->d_Wo2})
-        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, c->d_case_of, c->d_bmask, 0, c->d_case_W0, d);
+        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->d_case_of, c->d_bmask, 0, c->d_case_W0, d);
     return cuda_check(c, cudaGetLastError(), "reset");
 }
 
@@ -308,8 +321,7 @@ int batch_gmres(fp_ctx* c, const std::vector<int>& want, int kind, int m, int ma
     double* h2 = c->d_bcase + (size_t)(m + 1) * n;  // [m+1][n]
     double* nr = c->d_bcase + (size_t)2 * (m + 1) * n;
     const int* case_of = c->d_case_of;
-    const unsigned G = vgrid_of(nE);
-    const int K = c->nc;
+    const dim3 G = vgrid_of(nE, c->nc);
     int rc;
     if ((rc = cuda_check(c, cudaMemsetAsync(x, 0, N * sizeof(double), c->stream), "memset"))) return rc;
     // the kernels skip the elements of cases that are not iterating (live flags on the device,
@@ -352,7 +364,7 @@ int batch_gmres(fp_ctx* c, const std::vector<int>& want, int kind, int m, int ma
         // V_0 = r / ||r||_case
         if ((rc = set_live(active))) return rc;
         case_dots(c, r, nullptr, 1, nr);
-        k_case_normalise<<<G, 256, 0, c->stream>>>(nE, ld, K, case_of, c->d_blive, nr, r, V);
+        k_case_normalise<<<G, 256, 0, c->stream>>>(nE, ld, case_of, c->d_blive, nr, r, V);
         if ((rc = fetch_dev(c, nr, n, hh.data()))) return rc;
         std::vector<char> live(active);
         for (int cs = 0; cs < n; cs++) {
@@ -379,10 +391,10 @@ int batch_gmres(fp_ctx* c, const std::vector<int>& want, int kind, int m, int ma
             prof_begin(c, PH_KRYLOV);
             for (double* hk : {h1, h2}) {  // two classical Gram-Schmidt passes per case
                 case_dots(c, w, V, kc, hk);
-                k_case_maxpy<<<G, 256, 0, c->stream>>>(nE, ld, K, kc, n, case_of, c->d_blive, nullptr, -1.0, w, V, N, hk);
+                k_case_maxpy<<<G, 256, 0, c->stream>>>(nE, ld, kc, n, case_of, c->d_blive, nullptr, -1.0, w, V, N, hk);
             }
             case_dots(c, w, nullptr, 1, nr);
-            k_case_normalise<<<G, 256, 0, c->stream>>>(nE, ld, K, case_of, c->d_blive, nr, w, V + (size_t)(i + 1) * N);
+            k_case_normalise<<<G, 256, 0, c->stream>>>(nE, ld, case_of, c->d_blive, nr, w, V + (size_t)(i + 1) * N);
             prof_end(c);
             if ((rc = fetch_dev(c, c->d_bcase, (size_t)3 * (m + 1) * n, hh.data()))) return rc;
             for (int cs = 0; cs < n; cs++) {
@@ -432,14 +444,14 @@ int batch_gmres(fp_ctx* c, const std::vector<int>& want, int kind, int m, int ma
                 return rc;
             if ((rc = upload(c, c->d_bkc, kcs.data(), (size_t)n))) return rc;
             // each case's own Krylov vectors only (those past its count may be stale)
-            k_case_maxpy<<<G, 256, 0, c->stream>>>(nE, ld, K, kmax, n, case_of, c->d_blive, c->d_bkc, 1.0, x, V, N, h1);
+            k_case_maxpy<<<G, 256, 0, c->stream>>>(nE, ld, kmax, n, case_of, c->d_blive, c->d_bkc, 1.0, x, V, N, h1);
         }
         // true preconditioned residual per case
         prof_begin(c, PH_OPERATOR);
         rc = matfree_apply(c, x, aux);
         prof_end(c);
         if (rc) return rc;
-        k_bminus_all<<<G, 256, 0, c->stream>>>(N, aux, b);
+        k_bminus_all<<<(unsigned)std::min<size_t>((N + 255) / 256, 148 * 16), 256, 0, c->stream>>>(N, aux, b);
         if ((rc = prec_apply(c, kind, aux, r))) return rc;
         case_dots(c, r, nullptr, 1, nr);
         if ((rc = fetch_dev(c, nr, n, hh.data()))) return rc;
@@ -587,7 +599,7 @@ int fp_batch_solve(fp_ctx* c, const fp_implicit_params* pin, double* out, int* s
         {
             const int nch = c->batch_nch;
             k_chunk_min<<<nch, kRT, 0, c->stream>>>(nch, c->d_bch0, c->d_bch1, elem, c->d_bpart);
-            k_case_combine<<<(n + 127) / 128, 128, 0, c->stream>>>(n, c->d_bcptr, nch, 1, c->d_bpart, c->d_bcase, 1);
+            k_case_combine<<<combine_grid(n), 128, 0, c->stream>>>(n, c->d_bcptr, nch, 1, c->d_bpart, c->d_bcase, 1);
             hbuf.resize(n);
             if ((rc = fetch_dev(c, c->d_bcase, n, hbuf.data()))) return rc;
         }
@@ -652,9 +664,9 @@ int fp_batch_solve(fp_ctx* c, const fp_implicit_params* pin, double* out, int* s
                         st[cs].reduceCFL();
                         converges[cs] = 0;
                     }
-                const unsigned G = vgrid_of(c->hm.nElem);
+                const dim3 G = vgrid_of(c->hm.nElem, c->nc);
                 if ((rc = upload(c, c->d_bmask, back.data(), (size_t)n))) return rc;
-                k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, c->d_case_of, c->d_bmask, 0, c->d_Wo,
+                k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->d_case_of, c->d_bmask, 0, c->d_Wo,
                                                          c->d_W);
                 if ((rc = batch_reset(c, frozen))) return rc;
                 since = 1 << 30;
@@ -683,11 +695,11 @@ int fp_batch_solve(fp_ctx* c, const fp_implicit_params* pin, double* out, int* s
                 since = 1 << 30;  // the retry starts from a fresh preconditioner
             }
         }
-        const unsigned G = vgrid_of(c->hm.nElem);
+        const dim3 G = vgrid_of(c->hm.nElem, c->nc);
         if ((rc = upload(c, c->d_bmask, upd.data(), (size_t)n))) return rc;
-        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, c->d_case_of, c->d_bmask, 1, c->d_x, c->d_W);
+        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->d_case_of, c->d_bmask, 1, c->d_x, c->d_W);
         if ((rc = upload(c, c->d_bmask, back.data(), (size_t)n))) return rc;
-        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, c->d_case_of, c->d_bmask, 0, c->d_Wo, c->d_W);
+        k_case_masked<<<G, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->d_case_of, c->d_bmask, 0, c->d_Wo, c->d_W);
         if (c->hm.num.positivity_limiter && (rc = launch_positivity(c, c->d_W, nullptr))) return rc;
         if ((rc = fp_copy_w2wo(c))) return rc;
         for (int cs = 0; cs < n; cs++) {
