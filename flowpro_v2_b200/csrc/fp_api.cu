@@ -110,6 +110,8 @@ void free_all(fp_ctx* c) {
     c->allocs.clear();
     if (c->h_scal) cudaFreeHost(c->h_scal);
     c->h_scal = nullptr;
+    if (c->h_part) cudaFreeHost(c->h_part);
+    c->h_part = nullptr;
     c->d_Adiag = c->d_Aneigh = c->d_rhs = c->d_K0 = c->d_KR0 = c->d_P64 = nullptr;
     c->d_mass = nullptr;
     c->d_vu = nullptr;
@@ -451,12 +453,15 @@ int fp_mesh_upload(fp_ctx* c, const fp_mesh_desc* desc, const fp_model_params* m
         return rc;
     for (int i = 0; i < 3; i++)
         if ((rc = dalloc(c, &c->d_Wst[i], c->nvec))) return rc;
-    // partial sums: per-block reductions of the element kernels (8 per block of 128) and the
+    // partial sums: per-block reductions of the element kernels (up to 9 per block of 128) and the
     // fused Gram-Schmidt dots (592 blocks x up to 201 basis vectors)
-    size_t npart = std::max<size_t>((size_t)((h.nElem + 127) / 128) * 8, (size_t)592 * 201);
+    const size_t npelem = (size_t)((h.nElem + 127) / 128) * 9;
+    size_t npart = std::max<size_t>(npelem, (size_t)592 * 201);
     if ((rc = dalloc(c, &c->d_part, npart)) || (rc = dalloc(c, &c->d_scal, 1024)) || (rc = dalloc(c, &c->d_status, 4)))
         return rc;
-    if (cudaMallocHost(&c->h_scal, 1024 * sizeof(double)) != cudaSuccess) return set_err(c, FP_ERR_CUDA, "cudaMallocHost");
+    if (cudaMallocHost(&c->h_scal, 1024 * sizeof(double)) != cudaSuccess ||
+        cudaMallocHost(&c->h_part, npelem * sizeof(double)) != cudaSuccess)
+        return set_err(c, FP_ERR_CUDA, "cudaMallocHost");
     rc = cuda_check(c, cudaStreamSynchronize(c->stream), "upload sync");
     if (rc) return rc;
     c->has_mesh = true;
@@ -705,28 +710,41 @@ int fp_time_step_bound(fp_ctx* c, double* v) {
     return launch_dt_bound(c, v);
 }
 
-// RK3 stages 1-6 with the limiter before the residual stages and the positivity limiter
-// after the copy stages (LocalExplicitSolver.LocalTimeStepIterator.iterate, :267-288)
+}  // extern "C"
+
+namespace {
+
+// whether the limiter's values depend on the state; otherwise they are the same for every stage
+bool limiter_follows_state(const fp_ctx* c) { return c->hm.num.damp_tol > 0 && c->hm.num.order > 1; }
+
+// RK3 stages 1-5 with the limiter before the residual stages and the positivity limiter after the
+// copy stages (LocalExplicitSolver.LocalTimeStepIterator.iterate, :267-288), W -> W.  Each stage
+// writes the state the next one reads, so the copies of stages 2, 4 and 6 (W = W1, ...) are pointers:
+// the stage results stay as they are for the next combination, and with the positivity limiter the
+// limited state goes to a third array.  The positivity limiter of the last stage is left to the caller.
+int rk3_stages(fp_ctx* c, double dt) {
+    int rc;
+    double *W1 = c->d_Wst[0], *W2 = c->d_Wst[1], *Wl = c->d_Wst[2];
+    const bool pos = c->hm.num.positivity_limiter != 0, visc = limiter_follows_state(c);
+    // stage 1: W1 = Wo + dt M^-1 R(W), spatial residual kept
+    if ((rc = launch_rk_stage(c, c->d_W, c->d_Wo, c->d_Wo, 0.0, 1.0, dt, W1, c->d_R))) return rc;
+    if ((pos || visc) && (rc = launch_after_stage(c, W1, pos ? Wl : nullptr, visc))) return rc;
+    // stage 3: W2 = 3/4 Wo + 1/4 (W1 + dt M^-1 R(W))
+    if ((rc = launch_rk_stage(c, pos ? Wl : W1, c->d_Wo, W1, 0.75, 0.25, dt, W2, nullptr))) return rc;
+    if ((pos || visc) && (rc = launch_after_stage(c, W2, pos ? Wl : nullptr, visc))) return rc;
+    // stage 5: W = 1/3 Wo + 2/3 (W2 + dt M^-1 R(W))
+    return launch_rk_stage(c, pos ? Wl : W2, c->d_Wo, W2, 1.0 / 3, 2.0 / 3, dt, c->d_W, nullptr);
+}
+
+}  // namespace
+
+extern "C" {
+
 int fp_rk3_step(fp_ctx* c, double dt) {
     int rc = need_mesh(c);
     if (rc) return rc;
-    const size_t bytes = c->nvec * sizeof(double);
-    double *W1 = c->d_Wst[0], *W2 = c->d_Wst[1], *Wn = c->d_Wst[2];
-    const bool pos = c->hm.num.positivity_limiter != 0;
-    // stage 1: W1 = Wo + dt M^-1 R(W), spatial residual kept
-    if ((rc = launch_limiter(c)) || (rc = launch_rk_stage(c, c->d_W, c->d_Wo, c->d_Wo, 0.0, 1.0, dt, W1, c->d_R))) return rc;
-    // stage 2: W = W1
-    if ((rc = cuda_check(c, cudaMemcpyAsync(c->d_W, W1, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy"))) return rc;
-    if (pos && (rc = launch_positivity(c, c->d_W, nullptr))) return rc;
-    // stage 3: W2 = 3/4 Wo + 1/4 (W1 + dt M^-1 R(W))
-    if ((rc = launch_limiter(c)) || (rc = launch_rk_stage(c, c->d_W, c->d_Wo, W1, 0.75, 0.25, dt, W2, nullptr))) return rc;
-    if ((rc = cuda_check(c, cudaMemcpyAsync(c->d_W, W2, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy"))) return rc;
-    if (pos && (rc = launch_positivity(c, c->d_W, nullptr))) return rc;
-    // stage 5: Wn = 1/3 Wo + 2/3 (W2 + dt M^-1 R(W))
-    if ((rc = launch_limiter(c)) || (rc = launch_rk_stage(c, c->d_W, c->d_Wo, W2, 1.0 / 3, 2.0 / 3, dt, Wn, nullptr))) return rc;
-    if ((rc = cuda_check(c, cudaMemcpyAsync(c->d_W, Wn, bytes, cudaMemcpyDeviceToDevice, c->stream), "copy"))) return rc;
-    if (pos && (rc = launch_positivity(c, c->d_W, nullptr))) return rc;
-    return FP_OK;
+    if ((rc = launch_limiter(c)) || (rc = rk3_stages(c, dt))) return rc;
+    return c->hm.num.positivity_limiter ? launch_positivity(c, c->d_W, nullptr) : FP_OK;
 }
 
 int fp_copy_w2wo(fp_ctx* c) {
@@ -846,17 +864,22 @@ int fp_solve_explicit(fp_ctx* c, int steps, double cfl, double target, double* o
     st.vary = cfl <= 0;
     std::vector<double> norms(c->hm.model.n_eqs);
     const auto t_start = std::chrono::steady_clock::now();
+    double bound = 0;
     for (int s = 0; s < steps && st.residuum > target; s++) {
         st.steps++;
         st.updateCFL();
-        double bound = 0;
-        if ((rc = launch_dt_bound(c, &bound))) return rc;
+        if (s == 0 && (rc = launch_dt_bound(c, &bound))) return rc;
         double dt = st.currentCFL * bound;
-        if ((rc = fp_rk3_step(c, dt)) || (rc = launch_norms(c, c->d_R, norms.data()))) return rc;
+        if ((s == 0 || limiter_follows_state(c)) && (rc = launch_limiter(c))) return rc;
+        // the step, and in its last pass the state of the new time level (W -> Wo -> Wo2), the norms
+        // and the next step's bound
+        if ((rc = rk3_stages(c, dt)) ||
+            (rc = launch_step_end(c, c->hm.num.positivity_limiter != 0, c->d_Wo2, norms.data(), &bound)))
+            return rc;
+        std::swap(c->d_Wo, c->d_Wo2);
         st.setResiduum(norms);
         st.t += dt;
         st.dt = dt;
-        if ((rc = fp_copy_w2wo(c))) return rc;
         const bool stop = step_output(c, st, ms_since(t_start), &rc);
         if (rc) return rc;
         if (stop) break;

@@ -127,6 +127,7 @@ struct fp_ctx {
     double* d_part = nullptr;  // reduction partials
     double* d_scal = nullptr;  // device scalars
     double* h_scal = nullptr;  // pinned host mirror
+    double* h_part = nullptr;  // pinned host mirror of the partials of the element kernels
     unsigned* d_status = nullptr;
     // bookkeeping
     double last_dt = 0;
@@ -210,6 +211,8 @@ void pipe_release(fp_ctx* c);                                                   
 int launch_rk_stage(fp_ctx* c, const double* Wcur, const double* Wo, const double* Wb, double alpha, double beta, double dt,
                     double* Wout, double* Rsave);
 int launch_limiter(fp_ctx* c);
+int launch_after_stage(fp_ctx* c, const double* Win, double* Wout, bool visc);
+int launch_step_end(fp_ctx* c, bool pos, double* copy, double* norms, double* bound);
 int launch_positivity(fp_ctx* c, double* W, int* n_limited);
 int launch_norms(fp_ctx* c, const double* R, double* norms_host);
 int launch_dt_bound(fp_ctx* c, double* out_host);

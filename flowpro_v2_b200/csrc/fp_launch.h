@@ -8,6 +8,21 @@
 
 namespace fp {
 
+// arguments of the pass that follows an SSP-RK3 stage (null pointers: that part is left out)
+struct AfterStage {
+    const double* Win = nullptr;  // the stage's state
+    bool pos = false;             // positivity limiter, Win -> Wout
+    double* Wout = nullptr;
+    double* copy = nullptr;       // a copy of the (limited) state
+    double *eps = nullptr, *cip = nullptr;  // artificial viscosity and interior penalty of it
+    double dampTol = 0, penalty = 0;
+    const double* trun = nullptr;
+    const double* R = nullptr;    // partial norms of this residual
+    double* normPart = nullptr;
+    double factor = 1;            // partial time-step bounds of the state
+    double* dtPart = nullptr;
+};
+
 struct Launchers {
     int nc = 0;     // unknowns per element
     int ntrun = 0;  // size of the truncation matrix at the end of the reference tables
@@ -25,6 +40,7 @@ struct Launchers {
     void (*limiter)(const DevMesh&, cudaStream_t, const double* W, double dampTol, double penalty, const double* trun,
                     double* eps, double* cip) = nullptr;
     void (*positivity)(const DevMesh&, cudaStream_t, double* W, int* count) = nullptr;
+    void (*after_stage)(const DevMesh&, cudaStream_t, const AfterStage& A) = nullptr;
     void (*norms)(const DevMesh&, cudaStream_t, const double* R, double* part) = nullptr;
     void (*dtbound)(const DevMesh&, cudaStream_t, const double* W, double factor, double* part) = nullptr;
     void (*rhs)(const DevMesh&, cudaStream_t, const double* W, const double* Wo, const double* Wo2, double a1, double a2,

@@ -20,14 +20,28 @@ const Launchers* L(fp_ctx* c, int& rc) {
     return t;
 }
 
-int read_parts(fp_ctx* c, size_t n, std::vector<double>& h) {
-    h.resize(n);
-    int rc = cuda_check(c, cudaMemcpyAsync(h.data(), c->d_part, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "copy");
+// the first n partial sums on the host, in the context's pinned mirror of them
+int read_parts(fp_ctx* c, size_t n, const double*& h) {
+    int rc = cuda_check(c, cudaMemcpyAsync(c->h_part, c->d_part, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "copy");
     if (rc) return rc;
     rc = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
     prof_resolve(c);
+    h = c->h_part;
     return rc;
 }
+void norms_of_parts(const double* h, int nb, int ne, double* norms) {
+    for (int m = 0; m < ne; m++) {
+        double s = 0;
+        for (int b = 0; b < nb; b++) s += h[(size_t)b * ne + m];
+        norms[m] = std::sqrt(s);
+    }
+}
+double min_of_parts(const double* h, int nb) {
+    double m = 1.0e300;
+    for (int b = 0; b < nb; b++) m = std::min(m, h[b]);
+    return m;
+}
+double dt_factor(const fp_ctx* c) { return c->hm.num.implicit_time ? 1.0 : 2.0 * (c->hm.num.order - 1) + 1; }
 }  // namespace
 
 int launch_residual(fp_ctx* c, const double* W, double* R) {
@@ -280,6 +294,52 @@ int launch_limiter(fp_ctx* c) {
     return cuda_check(c, cudaGetLastError(), "limiter");
 }
 
+// the pass after an SSP-RK3 stage whose state is Win: the positivity limiter into Wout (null: none),
+// the artificial viscosity (visc), a copy of the state
+int launch_after_stage(fp_ctx* c, const double* Win, double* Wout, bool visc) {
+    int rc;
+    const Launchers* t = L(c, rc);
+    if (!t) return rc;
+    AfterStage a;
+    a.Win = Win;
+    a.pos = Wout != nullptr;
+    a.Wout = Wout;
+    if (visc) {
+        a.eps = c->d_eps;
+        a.cip = c->d_cip;
+        a.dampTol = c->hm.num.damp_tol;
+        a.penalty = c->hm.num.penalty;
+        a.trun = c->d_tab + c->hm.tab.data.size() - (size_t)t->ntrun;
+    }
+    t->after_stage(dev_mesh(c), c->stream, a);
+    return cuda_check(c, cudaGetLastError(), "after stage");
+}
+
+// the end of an explicit step: positivity limiter of W (pos), W -> copy, the norms of the spatial
+// residual and the time-step bound of W, fetched together
+int launch_step_end(fp_ctx* c, bool pos, double* copy, double* norms, double* bound) {
+    int rc;
+    const Launchers* t = L(c, rc);
+    if (!t) return rc;
+    const int nb = nblocks(c->hm.nElem), ne = c->hm.model.n_eqs;
+    AfterStage a;
+    a.Win = c->d_W;
+    a.pos = pos;
+    a.Wout = c->d_W;
+    a.copy = copy;
+    a.R = c->d_R;
+    a.normPart = c->d_part;
+    a.factor = dt_factor(c);
+    a.dtPart = c->d_part + (size_t)nb * ne;
+    t->after_stage(dev_mesh(c), c->stream, a);
+    if ((rc = cuda_check(c, cudaGetLastError(), "step end"))) return rc;
+    const double* h = nullptr;
+    if ((rc = read_parts(c, (size_t)nb * (ne + 1), h))) return rc;
+    norms_of_parts(h, nb, ne, norms);
+    *bound = min_of_parts(h + (size_t)nb * ne, nb);
+    return FP_OK;
+}
+
 int launch_positivity(fp_ctx* c, double* W, int* n_limited) {
     int rc;
     const Launchers* t = L(c, rc);
@@ -303,13 +363,9 @@ int launch_norms(fp_ctx* c, const double* R, double* norms) {
     t->norms(dev_mesh(c), c->stream, R, c->d_part);
     if ((rc = cuda_check(c, cudaGetLastError(), "norms"))) return rc;
     const int nb = nblocks(c->hm.nElem), ne = c->hm.model.n_eqs;
-    std::vector<double> h;
+    const double* h = nullptr;
     if ((rc = read_parts(c, (size_t)nb * ne, h))) return rc;
-    for (int m = 0; m < ne; m++) {
-        double s = 0;
-        for (int b = 0; b < nb; b++) s += h[(size_t)b * ne + m];
-        norms[m] = std::sqrt(s);
-    }
+    norms_of_parts(h, nb, ne, norms);
     return FP_OK;
 }
 
@@ -317,14 +373,11 @@ int launch_dt_bound(fp_ctx* c, double* out) {
     int rc;
     const Launchers* t = L(c, rc);
     if (!t) return rc;
-    const double factor = c->hm.num.implicit_time ? 1.0 : 2.0 * (c->hm.num.order - 1) + 1;
-    t->dtbound(dev_mesh(c), c->stream, c->d_W, factor, c->d_part);
+    t->dtbound(dev_mesh(c), c->stream, c->d_W, dt_factor(c), c->d_part);
     if ((rc = cuda_check(c, cudaGetLastError(), "dt bound"))) return rc;
-    std::vector<double> h;
+    const double* h = nullptr;
     if ((rc = read_parts(c, nblocks(c->hm.nElem), h))) return rc;
-    double m = 1.0e300;
-    for (double v : h) m = std::min(m, v);
-    *out = m;
+    *out = min_of_parts(h, nblocks(c->hm.nElem));
     return FP_OK;
 }
 
@@ -340,11 +393,9 @@ int launch_rhs(fp_ctx* c, double a1, double a2, double a3, double* rhs_norm) {
     prof_end(c);
     if ((rc = cuda_check(c, cudaGetLastError(), "rhs"))) return rc;
     if (!rhs_norm) return FP_OK;
-    std::vector<double> h;
+    const double* h = nullptr;
     if ((rc = read_parts(c, nblocks(c->hm.nElem), h))) return rc;
-    double s = 0;
-    for (double v : h) s += v;
-    *rhs_norm = std::sqrt(s);
+    norms_of_parts(h, nblocks(c->hm.nElem), 1, rhs_norm);
     return FP_OK;
 }
 
@@ -396,7 +447,7 @@ int launch_surface(fp_ctx* c, int kind, int bc, double* out4, double* dIdW) {
     t->surface(dev_mesh(c), c->stream, c->d_W, kind, bc, c->d_part, dIdW);
     if ((rc = cuda_check(c, cudaGetLastError(), "surface integral"))) return rc;
     const int nb = nblocks(c->hm.nElem);
-    std::vector<double> h;
+    const double* h = nullptr;
     if ((rc = read_parts(c, (size_t)nb * 4, h))) return rc;
     for (int v = 0; v < 4; v++) {
         double s = 0;

@@ -263,6 +263,66 @@ __global__ void __launch_bounds__(kBlock, (MinBlocks<Mdl, DIM, ORDER>::face))
     }
 }
 
+// The face pass of a mesh too small to fill the GPU with faces: one thread per face and quadrature
+// point (blockIdx.y), NQF times the threads, each of which reads the coefficients itself.  Up to
+// kFewFaces faces, two thread blocks of the other kernel per SM, a pass is bound by the length of one
+// thread's chain: 15,000 triangles p = 1 (22,700 faces) 13.0 -> 7.6 us.
+constexpr int kFewFaces = 2 * 148 * kBlock;
+struct OwnPlain {
+    const double* W;
+    size_t ld;
+    int e;
+    __device__ double operator[](int c) const { return ldg(W + c * ld + e); }
+};
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_face_points(DevMesh M, const double* __restrict__ W) {
+    using El = E<Mdl, DIM, ORDER>;
+    using GL = GeoLayout<DIM>;
+    constexpr int NE = El::NE, NQF = El::NQF, NP = El::NP;
+    const int f = blockIdx.x * blockDim.x + threadIdx.x, p = blockIdx.y;
+    const DevFaces& F = M.F;
+    if (f >= F.nFaces) return;
+    const int ld = M.ld, ldf = F.ldf;
+    const int e = F.fl[f], k = F.fk[f], TT = F.fr[f];
+    double n[DIM], Jac, dL;
+    El::face_geo(M, e, k, n, Jac, dL);
+    const bool interior = TT > -1;
+    int kr_face = 0, pm = 0;
+    double eps_nb = 0, cip_nb = 0;
+    if (interior) {
+        const int fc = F.fc[f];
+        kr_face = fc / NP;
+        pm = fc - kr_face * NP;
+        eps_nb = ldg(M.eps + TT);
+        cip_nb = ldg(M.cip + TT);
+    }
+    const double eps_e = ldg(M.eps + e), cip_e = ldg(M.cip + e);
+    const bool ip = Mdl::kViscous && (interior || Mdl::isIPFace(TT));
+    const OwnPlain w{W, (size_t)ld, e};
+    const NbPlain nbl{W, ld};
+    double Jinv[DIM * DIM], JinvR[DIM * DIM], C[NE], Jm[NE];
+    if (El::needs_gradients(M, interior, eps_e, eps_nb)) {
+#pragma unroll
+        for (int i = 0; i < DIM * DIM; i++) Jinv[i] = ldg(M.geo + (size_t)(GL::JINV + i) * ld + e);
+        if (interior) {
+#pragma unroll
+            for (int i = 0; i < DIM * DIM; i++) JinvR[i] = ldg(M.geo + (size_t)(GL::JINV + i) * ld + TT);
+        }
+        El::template face_point<true>(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+    } else if constexpr (!Mdl::kViscous) {
+        El::template face_point<false>(M, e, k, p, TT, n, dL, Jinv, JinvR, kr_face, pm, eps_e, eps_nb, w, nbl, C, Jm);
+    }
+    const double jw = Jac * ldg(M.tab + Tab<DIM, ORDER>::o_wf + p);
+    const int q = interior ? F.qmap[pm * NQF + p] : 0;
+    double* G0 = F.G + f;
+    double* G1 = F.G + (size_t)NQF * NE * ldf + f;
+#pragma unroll
+    for (int m = 0; m < NE; m++) {
+        G0[(size_t)(p * NE + m) * ldf] = jw * (ip ? C[m] - cip_e * Jm[m] : C[m]);
+        if (interior) G1[(size_t)(q * NE + m) * ldf] = jw * (ip ? -C[m] + cip_nb * Jm[m] : -C[m]);
+    }
+}
+
 template <class Mdl, int DIM, int ORDER>
 __global__ void __launch_bounds__(kBlock, (MinBlocks<Mdl, DIM, ORDER>::elem))
     k_residual(DevMesh M, const double* __restrict__ W, double* __restrict__ R, int e0, int e1) {
@@ -515,35 +575,40 @@ __global__ void __launch_bounds__(kBlock, 2)
 }
 
 // ---------------------------------------------------------------------------- limiter
+// integral means of the element's coefficients w (an array or an accessor)
+template <class Mdl, int DIM, int ORDER, class WA>
+__device__ __forceinline__ void element_means(const DevMesh& M, const WA& w, double* Ws) {
+    using TB = Tab<DIM, ORDER>;
+#pragma unroll
+    for (int m = 0; m < Mdl::NE; m++) {
+        double s = 0;
+#pragma unroll
+        for (int j = 0; j < TB::NB; j++) s = s + w[m * TB::NB + j] * ldg(M.tab + TB::o_Is + j);
+        Ws[m] = s;
+    }
+}
+
 // DGpure.limiter + shock_senzor (DGpure.java:358-452): eps = lambda h / order * sensor,
 // c_IP = penalty for diffusive models; both zero for piecewise constants.
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_limiter(DevMesh M, const double* __restrict__ W, double dampTol, double penalty, const double* __restrict__ trun,
-              double* __restrict__ eps, double* __restrict__ cip) {
+template <class Mdl, int DIM, int ORDER, class WA>
+__device__ __forceinline__ void limiter_values(const DevMesh& M, int e, const WA& w, double dampTol, double penalty,
+                                               const double* __restrict__ trun, double& ep, double& ci) {
     using TB = Tab<DIM, ORDER>;
     constexpr int NB = TB::NB, NE = Mdl::NE, NQV = TB::NQV;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M.nElem) return;
     const int ld = M.ld;
-    double ep = 0, ci = 0;
+    ep = 0;
+    ci = 0;
     if (ORDER > 1) {
-        double Ws[NE];
-#pragma unroll
-        for (int m = 0; m < NE; m++) {
-            double s = 0;
-#pragma unroll
-            for (int j = 0; j < NB; j++) s = s + ldg(W + (size_t)(m * NB + j) * ld + e) * ldg(M.tab + TB::o_Is + j);
-            Ws[m] = s;
-        }
-        double u[DIM];
-#pragma unroll
-        for (int d = 0; d < DIM; d++) u[d] = 0;
-        const double lam = val(Mdl::maxEigenvalue(Ws, u, M.P));
         if (dampTol > 0) {
+            double Ws[NE];
+            element_means<Mdl, DIM, ORDER>(M, w, Ws);
+            double u[DIM];
+#pragma unroll
+            for (int d = 0; d < DIM; d++) u[d] = 0;
+            const double lam = val(Mdl::maxEigenvalue(Ws, u, M.P));
             double rho[NB], tr[NB];
 #pragma unroll
-            for (int j = 0; j < NB; j++) rho[j] = ldg(W + (size_t)j * ld + e);
+            for (int j = 0; j < NB; j++) rho[j] = w[j];
             if (ORDER > 2) {
 #pragma unroll
                 for (int i = 0; i < NB; i++) {
@@ -584,6 +649,16 @@ __global__ void __launch_bounds__(kBlock)
         }
         if (Mdl::kViscous) ci = penalty;
     }
+}
+
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock)
+    k_limiter(DevMesh M, const double* __restrict__ W, double dampTol, double penalty, const double* __restrict__ trun,
+              double* __restrict__ eps, double* __restrict__ cip) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= M.nElem) return;
+    double ep, ci;
+    limiter_values<Mdl, DIM, ORDER>(M, e, OwnPlain{W, (size_t)M.ld, e}, dampTol, penalty, trun, ep, ci);
     eps[e] = ep;
     cip[e] = ci;
 }
@@ -617,129 +692,50 @@ __device__ double admissible_theta(const double* w, const double* Wavg, const do
     return lo;
 }
 
+// limits the coefficients w in place; true where it changed them
 template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock) k_positivity(DevMesh M, double* __restrict__ W, int* __restrict__ count) {
+__device__ __forceinline__ bool limit_positivity(const DevMesh& M, double* w) {
     using TB = Tab<DIM, ORDER>;
-    constexpr int NB = TB::NB, NE = Mdl::NE, NC = NE * NB;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M.nElem || NB == 1) return;
-    const int ld = M.ld;
-    double w[NC];
-    load_w<Mdl, DIM, ORDER>(W, ld, e, w);
+    constexpr int NB = TB::NB, NE = Mdl::NE;
+    if (NB == 1) return false;
     double Wavg[NE];
-#pragma unroll
-    for (int m = 0; m < NE; m++) {
-        double s = 0;
-#pragma unroll
-        for (int j = 0; j < NB; j++) s = s + w[m * NB + j] * ldg(M.tab + TB::o_Is + j);
-        Wavg[m] = s;
-    }
-    if (!Mdl::isAdmissible(Wavg)) return;
+    element_means<Mdl, DIM, ORDER>(M, w, Wavg);
+    if (!Mdl::isAdmissible(Wavg)) return false;
     double theta = 1;
     for (int q = 0; q < TB::NQV; q++) theta = fmin(theta, admissible_theta<Mdl, DIM, ORDER>(w, Wavg, M.tab + TB::o_phi + q * NB));
     for (int k = 0; k < TB::NF; k++)
         for (int p = 0; p < TB::NQF; p++)
             theta = fmin(theta, admissible_theta<Mdl, DIM, ORDER>(w, Wavg, M.tab + TB::o_phiL + (k * TB::NQF + p) * NB));
-    if (theta >= 1) return;
+    if (theta >= 1) return false;
 #pragma unroll
     for (int m = 0; m < NE; m++)
 #pragma unroll
         for (int i = 0; i < NB; i++) {
             const double mean = ldg(M.tab + TB::o_one + i) * Wavg[m];
-            W[(size_t)(m * NB + i) * ld + e] = mean + theta * (w[m * NB + i] - mean);
+            w[m * NB + i] = mean + theta * (w[m * NB + i] - mean);
         }
+    return true;
+}
+
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_positivity(DevMesh M, double* __restrict__ W, int* __restrict__ count) {
+    constexpr int NB = Tab<DIM, ORDER>::NB, NC = Mdl::NE * NB;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= M.nElem || NB == 1) return;
+    double w[NC];
+    load_w<Mdl, DIM, ORDER>(W, M.ld, e, w);
+    if (!limit_positivity<Mdl, DIM, ORDER>(M, w)) return;
+#pragma unroll
+    for (int c = 0; c < NC; c++) W[(size_t)c * M.ld + e] = w[c];
     atomicAdd(count, 1);
 }
 
 // ---------------------------------------------------------------------------- reductions
-// per-block partial sums of the element norms R_m^T M^-1 R_m (Element.l2NormsSquared)
+// element norms R_m^T M^-1 R_m (Element.l2NormsSquared)
 template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock) k_norms(DevMesh M, const double* __restrict__ R, double* __restrict__ part) {
+__device__ __forceinline__ void element_norms(const DevMesh& M, int e, const double* __restrict__ R, double* nrm) {
     using TB = Tab<DIM, ORDER>;
     constexpr int NB = TB::NB, NE = Mdl::NE;
-    __shared__ double sh[kBlock][NE];
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    double nrm[NE];
-#pragma unroll
-    for (int m = 0; m < NE; m++) nrm[m] = 0;
-    if (e < M.nElem) {
-        const int ld = M.ld;
-        const double ijac = 1.0 / ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
-#pragma unroll
-        for (int m = 0; m < NE; m++) {
-            double r[NB];
-#pragma unroll
-            for (int j = 0; j < NB; j++) r[j] = ldg(R + (size_t)(m * NB + j) * ld + e);
-            double sum = 0;
-#pragma unroll
-            for (int i = 0; i < NB; i++) {
-                double t = 0;
-#pragma unroll
-                for (int j = 0; j < NB; j++) t += ldg(M.tab + TB::o_MinvRef + i * NB + j) * ijac * r[j];
-                sum += r[i] * t;
-            }
-            nrm[m] = sum;
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < NE; m++) sh[threadIdx.x][m] = nrm[m];
-    __syncthreads();
-    for (int s = kBlock / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s)
-#pragma unroll
-            for (int m = 0; m < NE; m++) sh[threadIdx.x][m] += sh[threadIdx.x + s][m];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int m = 0; m < NE; m++) part[(size_t)blockIdx.x * NE + m] = sh[0][m];
-}
-
-// per-block minimum of elemSize / lambda (State.getTimeStep, Element.delta_t)
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock) k_dtbound(DevMesh M, const double* __restrict__ W, double factor, double* __restrict__ part) {
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NB = TB::NB, NE = Mdl::NE;
-    __shared__ double sh[kBlock];
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    double v = 1.0e300;
-    if (e < M.nElem) {
-        const int ld = M.ld;
-        double Ws[NE];
-#pragma unroll
-        for (int m = 0; m < NE; m++) {
-            double s = 0;
-#pragma unroll
-            for (int j = 0; j < NB; j++) s = s + ldg(W + (size_t)(m * NB + j) * ld + e) * ldg(M.tab + TB::o_Is + j);
-            Ws[m] = s;
-        }
-        double u[DIM];
-#pragma unroll
-        for (int d = 0; d < DIM; d++) {
-            u[d] = 0;
-            if (M.vu)
-                for (int v2 = 0; v2 < DIM + 1; v2++) u[d] += ldg(M.vu + (size_t)(v2 * DIM + d) * ld + e) / (DIM + 1);
-        }
-        const double lam = val(Mdl::maxEigenvalue(Ws, u, M.P));
-        if (lam > 0) v = ldg(M.geo + (size_t)GeoLayout<DIM>::SIZE * ld + e) / lam / factor;
-    }
-    sh[threadIdx.x] = v;
-    __syncthreads();
-    for (int s = kBlock / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) sh[threadIdx.x] = fmin(sh[threadIdx.x], sh[threadIdx.x + s]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
-}
-
-// per-element forms of the two reductions above, for a batch of cases (summed or minimised
-// per case afterwards): out[m][e] = R_m^T M^-1 R_m of element e, out[e] = elemSize / lambda / factor
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock) k_norms_elem(DevMesh M, const double* __restrict__ R, double* __restrict__ out) {
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NB = TB::NB, NE = Mdl::NE;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M.nElem) return;
     const int ld = M.ld;
     const double ijac = 1.0 / ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
 #pragma unroll
@@ -755,27 +751,16 @@ __global__ void __launch_bounds__(kBlock) k_norms_elem(DevMesh M, const double* 
             for (int j = 0; j < NB; j++) t += ldg(M.tab + TB::o_MinvRef + i * NB + j) * ijac * r[j];
             sum += r[i] * t;
         }
-        out[(size_t)m * ld + e] = sum;
+        nrm[m] = sum;
     }
 }
-
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_dtbound_elem(DevMesh M, const double* __restrict__ W, double factor, double* __restrict__ out) {
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NB = TB::NB, NE = Mdl::NE;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M.nElem) return;
+// elemSize / lambda / factor (State.getTimeStep, Element.delta_t) of the element's mean state
+template <class Mdl, int DIM, int ORDER, class WA>
+__device__ __forceinline__ double element_dt(const DevMesh& M, int e, const WA& w, double factor) {
+    constexpr int NE = Mdl::NE;
     const int ld = M.ld;
-    double v = 1.0e300;
     double Ws[NE];
-#pragma unroll
-    for (int m = 0; m < NE; m++) {
-        double s = 0;
-#pragma unroll
-        for (int j = 0; j < NB; j++) s = s + ldg(W + (size_t)(m * NB + j) * ld + e) * ldg(M.tab + TB::o_Is + j);
-        Ws[m] = s;
-    }
+    element_means<Mdl, DIM, ORDER>(M, w, Ws);
     double u[DIM];
 #pragma unroll
     for (int d = 0; d < DIM; d++) {
@@ -784,8 +769,114 @@ __global__ void __launch_bounds__(kBlock)
             for (int v2 = 0; v2 < DIM + 1; v2++) u[d] += ldg(M.vu + (size_t)(v2 * DIM + d) * ld + e) / (DIM + 1);
     }
     const double lam = val(Mdl::maxEigenvalue(Ws, u, M.P));
-    if (lam > 0) v = ldg(M.geo + (size_t)GeoLayout<DIM>::SIZE * ld + e) / lam / factor;
-    out[e] = v;
+    return lam > 0 ? ldg(M.geo + (size_t)GeoLayout<DIM>::SIZE * ld + e) / lam / factor : 1.0e300;
+}
+// the block's sums of nrm[0 .. NE - 1] into part[block * NE + m], the same tree for any caller
+template <int NE>
+__device__ __forceinline__ void block_sums(const double* nrm, double* part) {
+    __shared__ double sh[kBlock][NE];
+#pragma unroll
+    for (int m = 0; m < NE; m++) sh[threadIdx.x][m] = nrm[m];
+    __syncthreads();
+    for (int s = kBlock / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s)
+#pragma unroll
+            for (int m = 0; m < NE; m++) sh[threadIdx.x][m] += sh[threadIdx.x + s][m];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int m = 0; m < NE; m++) part[(size_t)blockIdx.x * NE + m] = sh[0][m];
+}
+__device__ __forceinline__ void block_min(double v, double* part) {
+    __shared__ double sh[kBlock];
+    sh[threadIdx.x] = v;
+    __syncthreads();
+    for (int s = kBlock / 2; s > 0; s >>= 1) {
+        if ((int)threadIdx.x < s) sh[threadIdx.x] = fmin(sh[threadIdx.x], sh[threadIdx.x + s]);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
+}
+
+// per-block partial sums of the element norms
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_norms(DevMesh M, const double* __restrict__ R, double* __restrict__ part) {
+    constexpr int NE = Mdl::NE;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    double nrm[NE];
+#pragma unroll
+    for (int m = 0; m < NE; m++) nrm[m] = 0;
+    if (e < M.nElem) element_norms<Mdl, DIM, ORDER>(M, e, R, nrm);
+    block_sums<NE>(nrm, part);
+}
+
+// per-block minimum of elemSize / lambda
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_dtbound(DevMesh M, const double* __restrict__ W, double factor, double* __restrict__ part) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    block_min(e < M.nElem ? element_dt<Mdl, DIM, ORDER>(M, e, OwnPlain{W, (size_t)M.ld, e}, factor) : 1.0e300, part);
+}
+
+// What follows an SSP-RK3 stage, in one pass over the elements instead of a kernel or a copy each:
+// the positivity limiter (A.pos: Win -> Wout, the same array or another one), the artificial viscosity
+// of the state (A.eps), a copy of it (A.copy), and at the end of a step the partial norms of the
+// spatial residual R and the partial time-step bounds of the new state.
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_after_stage(DevMesh M, AfterStage A) {
+    using TB = Tab<DIM, ORDER>;
+    constexpr int NE = Mdl::NE, NC = NE * TB::NB;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    double nrm[NE], dt = 1.0e300;
+#pragma unroll
+    for (int m = 0; m < NE; m++) nrm[m] = 0;
+    if (e < M.nElem) {
+        const int ld = M.ld;
+        if (A.pos || A.copy || A.eps || A.dtPart) {
+            double w[NC];
+#pragma unroll
+            for (int c = 0; c < NC; c++) w[c] = A.Win[(size_t)c * ld + e];
+            if (A.pos) {
+                limit_positivity<Mdl, DIM, ORDER>(M, w);
+#pragma unroll
+                for (int c = 0; c < NC; c++) A.Wout[(size_t)c * ld + e] = w[c];
+            }
+            if (A.copy) {
+#pragma unroll
+                for (int c = 0; c < NC; c++) A.copy[(size_t)c * ld + e] = w[c];
+            }
+            if (A.eps) {
+                double ep, ci;
+                limiter_values<Mdl, DIM, ORDER>(M, e, w, A.dampTol, A.penalty, A.trun, ep, ci);
+                A.eps[e] = ep;
+                A.cip[e] = ci;
+            }
+            if (A.dtPart) dt = element_dt<Mdl, DIM, ORDER>(M, e, w, A.factor);
+        }
+        if (A.normPart) element_norms<Mdl, DIM, ORDER>(M, e, A.R, nrm);
+    }
+    if (A.normPart) block_sums<NE>(nrm, A.normPart);
+    if (A.dtPart) block_min(dt, A.dtPart);
+}
+
+// per-element forms of the two reductions above, for a batch of cases (summed or minimised
+// per case afterwards): out[m][e] = R_m^T M^-1 R_m of element e, out[e] = elemSize / lambda / factor
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock) k_norms_elem(DevMesh M, const double* __restrict__ R, double* __restrict__ out) {
+    constexpr int NE = Mdl::NE;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= M.nElem) return;
+    double nrm[NE];
+    element_norms<Mdl, DIM, ORDER>(M, e, R, nrm);
+#pragma unroll
+    for (int m = 0; m < NE; m++) out[(size_t)m * M.ld + e] = nrm[m];
+}
+
+template <class Mdl, int DIM, int ORDER>
+__global__ void __launch_bounds__(kBlock)
+    k_dtbound_elem(DevMesh M, const double* __restrict__ W, double factor, double* __restrict__ out) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < M.nElem) out[e] = element_dt<Mdl, DIM, ORDER>(M, e, OwnPlain{W, (size_t)M.ld, e}, factor);
 }
 
 // ---------------------------------------------------------------------------- implicit RHS
@@ -1382,7 +1473,10 @@ struct Launch {
     }
     static void faces(const DevMesh& M, cudaStream_t s, const double* W) {
         prepare();
-        k_face<Mdl, DIM, ORDER><<<grid_of(M.F.nFaces), kBlock, kDynFace, s>>>(M, W, 0, M.F.nFaces);
+        if (M.F.nFaces <= kFewFaces && Element<Mdl, DIM, ORDER>::NQF > 1)
+            k_face_points<Mdl, DIM, ORDER><<<dim3(grid_of(M.F.nFaces), Element<Mdl, DIM, ORDER>::NQF), kBlock, 0, s>>>(M, W);
+        else
+            k_face<Mdl, DIM, ORDER><<<grid_of(M.F.nFaces), kBlock, kDynFace, s>>>(M, W, 0, M.F.nFaces);
     }
     static void elements(const DevMesh& M, cudaStream_t s, const double* W, double* R) {
         prepare();
@@ -1424,6 +1518,9 @@ struct Launch {
     }
     static void positivity(const DevMesh& M, cudaStream_t s, double* W, int* count) {
         k_positivity<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, W, count);
+    }
+    static void after_stage(const DevMesh& M, cudaStream_t s, const AfterStage& A) {
+        k_after_stage<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, A);
     }
     static void norms(const DevMesh& M, cudaStream_t s, const double* R, double* part) {
         k_norms<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, R, part);
@@ -1493,6 +1590,7 @@ struct Launch {
         t.matfree_gather = matfree_gather;
         t.limiter = limiter;
         t.positivity = positivity;
+        t.after_stage = after_stage;
         t.norms = norms;
         t.dtbound = dtbound;
         t.rhs = rhs;
