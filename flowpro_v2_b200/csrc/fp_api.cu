@@ -157,7 +157,7 @@ __global__ void k_from_soa(int nElem, int ld, int nc, const double* __restrict__
 
 int host_to_soa(fp_ctx* c, const double* h, double* d) {
     size_t n = (size_t)c->hm.nElem * c->nc;
-    int rc = upload(c, c->d_io, h, n);
+    int rc = copy_to_device(c, c->d_io, h, n * sizeof(double));
     if (rc) return rc;
     k_to_soa<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, c->d_io, d);
     return cuda_check(c, cudaGetLastError(), "to soa");
@@ -168,9 +168,7 @@ int soa_to_host(fp_ctx* c, const double* d, double* h) {
     k_from_soa<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->nc, d, c->d_io);
     int rc = cuda_check(c, cudaGetLastError(), "from soa");
     if (rc) return rc;
-    rc = cuda_check(c, cudaMemcpyAsync(h, c->d_io, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "download");
-    if (rc) return rc;
-    return cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
+    return copy_to_host(c, h, c->d_io, n * sizeof(double));
 }
 
 int need_mesh(fp_ctx* c) {
@@ -287,6 +285,7 @@ int fp_ctx_create(int device, fp_ctx** out) {
         delete c;
         return FP_ERR_CUDA;
     }
+    staging_retain();
     *out = c;
     return FP_OK;
 }
@@ -302,6 +301,7 @@ int fp_ctx_destroy(fp_ctx* c) {
     if (c->s_d2h) cudaStreamDestroy(c->s_d2h);
     if (c->s_elem) cudaStreamDestroy(c->s_elem);
     if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
+    staging_release();
     delete c;
     return FP_OK;
 }

@@ -210,6 +210,12 @@ int launch_residual_pipelined(fp_ctx* c, const double* w_host, double* r_host); 
 void pipe_release(fp_ctx* c);                                                        // drop the captured sequence
 int launch_rk_stage(fp_ctx* c, const double* Wcur, const double* Wo, const double* Wb, double alpha, double beta, double dt,
                     double* Wout, double* Rsave);
+// host copies on the context's stream (fp_hostcopy.cu); copy_to_host has finished on return, the source of
+// copy_to_device may be reused once the stream has passed it (at once where it is pageable)
+void staging_retain();
+void staging_release();
+int copy_to_host(fp_ctx* c, void* host, const void* dev, size_t bytes);
+int copy_to_device(fp_ctx* c, void* dev, const void* host, size_t bytes);
 int launch_limiter(fp_ctx* c);
 int launch_after_stage(fp_ctx* c, const double* Win, double* Wout, bool visc);
 int launch_step_end(fp_ctx* c, bool pos, double* copy, double* norms, double* bound);
