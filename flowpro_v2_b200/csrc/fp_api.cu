@@ -90,6 +90,7 @@ DevMesh dev_mesh(const fp_ctx* c) {
     M.ncases = c->n_cases;
     M.case_live = (c->n_cases > 0 && c->batch_mask) ? c->d_blive : nullptr;
     M.dampConst = c->hm.num.damp_const;
+    M.artificial = c->hm.num.damp_tol > 0 || c->hm.num.damp_const != 0;
     // DGpure.residuumWall sets beta0 = 0 for a global order 1 with a diffusive model (DGpure.java:287-289)
     M.beta0 = (c->hm.model.is_diffusive && c->hm.num.order == 1) ? 0.0 : c->hm.num.beta0;
     M.P = c->hm.model;

@@ -72,6 +72,7 @@ struct DevMesh {
     const int* __restrict__ case_live;
     int ncases;
     double dampConst, beta0;
+    bool artificial;  // an element may carry artificial viscosity (eps or dampConst not zero)
     fp_model_params P;
     DevFaces F;
 };
@@ -406,48 +407,108 @@ struct Element {
         volume(M, e, w, Jinv, eps_e, K);
     }
 
-    // volume integral of DGpure.residuum (DGpure.java:116-191)
-    template <class T, class WA>
-    static __device__ __forceinline__ void volume(const DevMesh& M, int e, const WA& w, const double* Jinv, double eps_e,
-                                                  T* K) {
+    // Integrand of the volume integral at quadrature point q from the state WI and its gradient dWI:
+    // Gr[dp * NE + m], the weighted coefficients of the basis functions' reference gradients, and s[m], the
+    // weighted source
+    template <class T>
+    static __device__ __forceinline__ void volume_point(const DevMesh& M, int e, int q, const double* Jinv, double jw, double avc,
+                                                        T* WI, T* dWI, T* Gr, T* sw) {
         const int ld = M.ld;
         const double* geo = M.geo;
         const double* tab = M.tab;
         const fp_model_params& P = M.P;
         const bool volumeFluxes = ORDER > 1;
+        double u[DIM];
+#pragma unroll
+        for (int d = 0; d < DIM; d++) u[d] = 0;
+        double D = 0, X[DIM];
+        if (M.vu != nullptr) {
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                const double li = ldg(tab + TB::o_interp + q * NV + v);
+#pragma unroll
+                for (int d = 0; d < DIM; d++) u[d] += li * ldg(M.vu + (size_t)(v * DIM + d) * ld + e);
+            }
+        }
+        if (Mdl::kSource) {
+#pragma unroll
+            for (int v = 0; v < NV; v++) D += ldg(tab + TB::o_interp + q * NV + v) * ldg(M.vwd + (size_t)v * ld + e);
+            const double* xi = tab + TB::o_xi + q * DIM;
+#pragma unroll
+            for (int i = 0; i < DIM; i++) {
+                double s = 0;
+#pragma unroll
+                for (int j = 0; j < DIM; j++) s += ldg(geo + (size_t)(GL::JM + i * DIM + j) * ld + e) * ldg(xi + j);
+                X[i] = s + ldg(geo + (size_t)(GL::X0 + i) * ld + e);
+            }
+        }
+        // G[d][m]: coefficient of d(phi_j)/dx_d, then mapped to the reference gradient
+        T G[DIM * NE];
+#pragma unroll
+        for (int i = 0; i < DIM * NE; i++) G[i] = 0.0;
+        // fast path when no density limiting can occur (bit-identical to the per-axis calls)
+        const bool unlimited = val(WI[0]) >= RHO_TOL;
+        if (volumeFluxes && Mdl::kConvective) {
+            if (unlimited) {
+                Mdl::convectiveFluxAll(WI, G, P);
+            } else {
+#pragma unroll
+                for (int d = 0; d < DIM; d++) {
+                    T f[NE];
+                    Mdl::convectiveFluxAxis(WI, d, f, P);
+#pragma unroll
+                    for (int m = 0; m < NE; m++) G[d * NE + m] = f[m];
+                }
+            }
+        }
+        if (volumeFluxes && Mdl::kViscous) {
+            T fv[DIM * NE];
+            if (unlimited) {
+                Mdl::diffusiveFluxAll(WI, dWI, fv, P);
+            } else {
+#pragma unroll
+                for (int d = 0; d < DIM; d++) Mdl::diffusiveFlux(WI, dWI, (const double*)nullptr, d, fv + d * NE, P);
+            }
+#pragma unroll
+            for (int i = 0; i < DIM * NE; i++) G[i] -= fv[i];
+        }
+        T s[NE];
+        if (Mdl::kSource) Mdl::sourceTerm(WI, dWI, D, X, s, P);
+        if (volumeFluxes) {
+#pragma unroll
+            for (int d = 0; d < DIM; d++)
+#pragma unroll
+                for (int m = 0; m < NE; m++) G[d * NE + m] = jw * (G[d * NE + m] - u[d] * WI[m] - avc * dWI[d * NE + m]);
+#pragma unroll
+            for (int m = 0; m < NE; m++)
+#pragma unroll
+                for (int dp = 0; dp < DIM; dp++) {
+                    T t = 0.0;
+#pragma unroll
+                    for (int d = 0; d < DIM; d++) t += Jinv[dp * DIM + d] * G[d * NE + m];
+                    Gr[dp * NE + m] = t;
+                }
+        }
+        if (Mdl::kSource) {
+#pragma unroll
+            for (int m = 0; m < NE; m++) sw[m] = jw * s[m];
+        }
+    }
+
+    // volume integral of DGpure.residuum (DGpure.java:116-191)
+    template <class T, class WA>
+    static __device__ __forceinline__ void volume(const DevMesh& M, int e, const WA& w, const double* Jinv, double eps_e,
+                                                  T* K) {
+        const double* tab = M.tab;
+        const bool volumeFluxes = ORDER > 1;
         if (!(volumeFluxes || Mdl::kSource)) return;
-        const double jac = ldg(geo + (size_t)GL::JAC * ld + e);
+        const double jac = ldg(M.geo + (size_t)GL::JAC * M.ld + e);
         const double avc = eps_e + M.dampConst;
 #pragma unroll 1
         for (int q = 0; q < NQV; q++) {
-            const double weight = ldg(tab + TB::o_w + q);
             const double* phi = tab + TB::o_phi + q * NB;
             const double* dphi = tab + TB::o_dphi + q * NB * DIM;
-            double u[DIM];
-#pragma unroll
-            for (int d = 0; d < DIM; d++) u[d] = 0;
-            double D = 0, X[DIM];
-            if (M.vu != nullptr) {
-#pragma unroll
-                for (int v = 0; v < NV; v++) {
-                    const double li = ldg(tab + TB::o_interp + q * NV + v);
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) u[d] += li * ldg(M.vu + (size_t)(v * DIM + d) * ld + e);
-                }
-            }
-            if (Mdl::kSource) {
-#pragma unroll
-                for (int v = 0; v < NV; v++) D += ldg(tab + TB::o_interp + q * NV + v) * ldg(M.vwd + (size_t)v * ld + e);
-                const double* xi = tab + TB::o_xi + q * DIM;
-#pragma unroll
-                for (int i = 0; i < DIM; i++) {
-                    double s = 0;
-#pragma unroll
-                    for (int j = 0; j < DIM; j++) s += ldg(geo + (size_t)(GL::JM + i * DIM + j) * ld + e) * ldg(xi + j);
-                    X[i] = s + ldg(geo + (size_t)(GL::X0 + i) * ld + e);
-                }
-            }
-            T WI[NE], dWI[DIM * NE];
+            T WI[NE], dWI[DIM * NE], Gr[DIM * NE], sw[NE];
             if (Mdl::kViscous || Mdl::kSource || avc != 0.0) {
                 trace<true>(phi, dphi, Jinv, [&](int c) { return w[c]; }, WI, dWI);
             } else {  // nothing reads the gradient: its coefficient is exactly zero
@@ -455,69 +516,21 @@ struct Element {
 #pragma unroll
                 for (int i = 0; i < DIM * NE; i++) dWI[i] = 0.0;
             }
-            const double jw = jac * weight;
-            // G[d][m]: coefficient of d(phi_j)/dx_d, then mapped to the reference gradient
-            T G[DIM * NE];
+            volume_point(M, e, q, Jinv, jac * ldg(tab + TB::o_w + q), avc, WI, dWI, Gr, sw);
 #pragma unroll
-            for (int i = 0; i < DIM * NE; i++) G[i] = 0.0;
-            // fast path when no density limiting can occur (bit-identical to the per-axis calls)
-            const bool unlimited = val(WI[0]) >= RHO_TOL;
-            if (volumeFluxes && Mdl::kConvective) {
-                if (unlimited) {
-                    Mdl::convectiveFluxAll(WI, G, P);
-                } else {
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) {
-                        T f[NE];
-                        Mdl::convectiveFluxAxis(WI, d, f, P);
-#pragma unroll
-                        for (int m = 0; m < NE; m++) G[d * NE + m] = f[m];
-                    }
-                }
-            }
-            if (volumeFluxes && Mdl::kViscous) {
-                T fv[DIM * NE];
-                if (unlimited) {
-                    Mdl::diffusiveFluxAll(WI, dWI, fv, P);
-                } else {
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) Mdl::diffusiveFlux(WI, dWI, (const double*)nullptr, d, fv + d * NE, P);
-                }
-#pragma unroll
-                for (int i = 0; i < DIM * NE; i++) G[i] -= fv[i];
-            }
-            T s[NE];
-            if (Mdl::kSource) Mdl::sourceTerm(WI, dWI, D, X, s, P);
-            if (volumeFluxes) {
-#pragma unroll
-                for (int d = 0; d < DIM; d++)
-#pragma unroll
-                    for (int m = 0; m < NE; m++) G[d * NE + m] = jw * (G[d * NE + m] - u[d] * WI[m] - avc * dWI[d * NE + m]);
-#pragma unroll
-                for (int m = 0; m < NE; m++) {
-                    T Gr[DIM];
-#pragma unroll
-                    for (int dp = 0; dp < DIM; dp++) {
-                        T t = 0.0;
-#pragma unroll
-                        for (int d = 0; d < DIM; d++) t += Jinv[dp * DIM + d] * G[d * NE + m];
-                        Gr[dp] = t;
-                    }
+            for (int m = 0; m < NE; m++) {
+                if (volumeFluxes) {
 #pragma unroll
                     for (int j = 0; j < NB; j++) {
                         T a = K[m * NB + j];
 #pragma unroll
-                        for (int dp = 0; dp < DIM; dp++) a += Gr[dp] * ldg(dphi + j * DIM + dp);
+                        for (int dp = 0; dp < DIM; dp++) a += Gr[dp * NE + m] * ldg(dphi + j * DIM + dp);
                         K[m * NB + j] = a;
                     }
                 }
-            }
-            if (Mdl::kSource) {
+                if (Mdl::kSource) {
 #pragma unroll
-                for (int m = 0; m < NE; m++) {
-                    const T sw = jw * s[m];
-#pragma unroll
-                    for (int j = 0; j < NB; j++) K[m * NB + j] += sw * ldg(phi + j);
+                    for (int j = 0; j < NB; j++) K[m * NB + j] += sw[m] * ldg(phi + j);
                 }
             }
         }

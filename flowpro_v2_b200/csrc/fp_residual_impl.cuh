@@ -1045,128 +1045,6 @@ __global__ void __launch_bounds__(kBlock)
     }
 }
 
-// ---------------------------------------------------------------------------- exact element Jacobian
-// The FD assembly above with the finite difference replaced by the exact tangent: column i
-// of the blocks is the Dual<1> derivative of the element residual (and of this element's
-// face contributions to its neighbours) along e_i.  Same storage and signs as k_fd_col.
-template <int N>
-struct NbConst {
-    const double* W;
-    int ld;
-    __device__ Dual<N> operator()(int c, int nb) const { return Dual<N>(ldg(W + (size_t)c * ld + nb)); }
-};
-
-template <int NC>
-struct KRColExact {
-    static constexpr bool enabled = true;
-    double acc[NC];
-    double* Aneigh;
-    int ld, i;
-    template <class T>
-    __device__ void begin(int) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) acc[c] = 0;
-    }
-    __device__ void add(int, int c, const Dual<1>& v) { acc[c] += v.d[0]; }
-    __device__ void end(int, int nb, int kr) {
-        double* A = Aneigh + (size_t)kr * NC * NC * ld;
-#pragma unroll
-        for (int r = 0; r < NC; r++) A[((size_t)r * NC + i) * ld + nb] = acc[r];
-    }
-};
-
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_jac_exact(DevMesh M, const double* __restrict__ W, double a1, double* __restrict__ Adiag, double* __restrict__ Aneigh) {
-    using El = E<Mdl, DIM, ORDER>;
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NC = El::NC, NB = El::NB;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t % M.nElem);
-    const int i = (int)(t / M.nElem);
-    if (i >= NC) return;
-    case_coefficients(M, e, a1);
-    const int ld = M.ld;
-    Dual<1> w[NC], K[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        w[c].v = ldg(W + (size_t)c * ld + e);
-        w[c].d[0] = c == i ? 1.0 : 0.0;
-    }
-    KRColExact<NC> kr;
-    kr.Aneigh = Aneigh;
-    kr.ld = ld;
-    kr.i = i;
-    El::residual(M, e, w, NbConst<1>{W, ld}, K, kr);
-    const double jac = ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
-    const int mi = i / NB, bi = i - mi * NB;
-#pragma unroll
-    for (int r = 0; r < NC; r++) {
-        double a = -K[r].d[0];
-        const int mr = r / NB, br = r - mr * NB;
-        if (mr == mi) a += a1 * mass_entry<DIM, ORDER>(M, e, 0, br, bi, jac);
-        Adiag[((size_t)r * NC + i) * ld + e] = a;
-    }
-}
-
-// The exact blocks written straight into the block ILU(0) factor storage (element-major,
-// column-major blocks F[e][s][c][r] in T = float or double; s = 0 the diagonal block, s = 1 + k
-// the block coupling the row element with its neighbour over face k), so the matrix-free
-// Newton path keeps no copy of the operator's blocks: column i of element e's diagonal block
-// and column i of each neighbour's block toward e, each a contiguous run of NC values.
-template <int NC, int NF, class T>
-struct KRColFactor {
-    static constexpr bool enabled = true;
-    double acc[NC];
-    T* F;
-    int i;
-    template <class U>
-    __device__ void begin(int) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) acc[c] = 0;
-    }
-    __device__ void add(int, int c, const Dual<1>& v) { acc[c] += v.d[0]; }
-    __device__ void end(int, int nb, int kr) {
-        T* A = F + (((size_t)nb * (1 + NF) + 1 + kr) * NC + i) * NC;
-#pragma unroll
-        for (int r = 0; r < NC; r++) A[r] = (T)acc[r];
-    }
-};
-
-template <class Mdl, int DIM, int ORDER, class T>
-__global__ void __launch_bounds__(kBlock)
-    k_jac_exact_factor(DevMesh M, const double* __restrict__ W, double a1, T* __restrict__ F) {
-    using El = E<Mdl, DIM, ORDER>;
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NC = El::NC, NB = El::NB, NF = El::NF;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t % M.nElem);
-    const int i = (int)(t / M.nElem);
-    if (i >= NC) return;
-    case_coefficients(M, e, a1);
-    const int ld = M.ld;
-    Dual<1> w[NC], K[NC];
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        w[c].v = ldg(W + (size_t)c * ld + e);
-        w[c].d[0] = c == i ? 1.0 : 0.0;
-    }
-    KRColFactor<NC, NF, T> kr;
-    kr.F = F;
-    kr.i = i;
-    El::residual(M, e, w, NbConst<1>{W, ld}, K, kr);
-    const double jac = ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
-    const int mi = i / NB, bi = i - mi * NB;
-    T* A = F + ((size_t)e * (1 + NF) * NC + i) * NC;
-#pragma unroll
-    for (int r = 0; r < NC; r++) {
-        double a = -K[r].d[0];
-        const int mr = r / NB, br = r - mr * NB;
-        if (mr == mi) a += a1 * mass_entry<DIM, ORDER>(M, e, 0, br, bi, jac);
-        A[r] = (T)a;
-    }
-}
-
 // ---------------------------------------------------------------------------- moving mesh
 // Mass matrix of time level lev from the current geometry (DGpure.recalculateMassMatrix,
 // DGpure.java:575-593): M_ij = sum_p jac w_p phi_i(p) phi_j(p), in the reference's order.
@@ -1270,57 +1148,27 @@ __global__ void __launch_bounds__(kBlock) k_gcl_mass(DevMesh M, double a1, doubl
         }
 }
 
-// ---------------------------------------------------------------------------- VJP
-// g = (dR/dW)^T lambda without a stored Jacobian: thread (e, i) forms column i of its
-// element's blocks in registers (the Dual<1> tangent of the element residual along e_i,
-// quadrature states recomputed, as k_jac_exact does) and contracts it at once with the
-// adjoint weights it multiplies: lambda_e for the element's own rows and lambda_nb for the rows
-// of each face neighbour its face integrals feed (the KR terms of DGpure.residuumWall), so
-// g[i][e] = sum_r dR_e[r]/dW_e,i lambda_e[r] + sum_nb sum_r dR_nb[r]/dW_e,i lambda_nb[r].
-// The neighbour terms carry the sign of the assembled neighbour blocks (A = a1 M - dR/dW).
-struct KRColVjp {
-    static constexpr bool enabled = true;
-    const int* tt;
-    const double* lam;
-    int ld, e, nb;
-    double s;
-    template <class U>
-    __device__ void begin(int k) {
-        nb = tt[(size_t)k * ld + e];
-    }
-    __device__ void add(int, int c, const Dual<1>& v) { s += v.d[0] * ldg(lam + (size_t)c * ld + nb); }
-    __device__ void end(int, int, int) {}
-};
-
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_vjp_cols(DevMesh M, const double* __restrict__ W, const double* __restrict__ lam, double* __restrict__ g) {
-    using El = E<Mdl, DIM, ORDER>;
-    constexpr int NC = El::NC;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t % M.nElem);
-    const int i = (int)(t / M.nElem);
-    if (i >= NC) return;
-    const int ld = M.ld;
-    Dual<1> w[NC], K[NC];
+// a contiguous column of NC values, two at a time where their address allows it
+template <int NC, class T>
+__device__ __forceinline__ void store_column(T* dst, const double* v) {
+    if constexpr (NC % 2 == 0) {
+        using T2 = std::conditional_t<sizeof(T) == 8, double2, float2>;
 #pragma unroll
-    for (int c = 0; c < NC; c++) {
-        w[c].v = ldg(W + (size_t)c * ld + e);
-        w[c].d[0] = c == i ? 1.0 : 0.0;
-    }
-    KRColVjp kr;
-    kr.tt = M.tt;
-    kr.lam = lam;
-    kr.ld = ld;
-    kr.e = e;
-    kr.nb = -1;
-    kr.s = 0.0;
-    El::residual(M, e, w, NbConst<1>{W, ld}, K, kr);
-    double own = 0.0;
+        for (int r = 0; r < NC; r += 2) {
+            T2 x;
+            x.x = (T)v[r];
+            x.y = (T)v[r + 1];
+            reinterpret_cast<T2*>(dst)[r / 2] = x;
+        }
+    } else {
 #pragma unroll
-    for (int r = 0; r < NC; r++) own += K[r].d[0] * ldg(lam + (size_t)r * ld + e);
-    g[(size_t)i * ld + e] = own - kr.s;
+        for (int r = 0; r < NC; r++) dst[r] = (T)v[r];
+    }
 }
+
+}  // namespace fp
+#include "fp_jacobian.cuh"
+namespace fp {
 
 // ---------------------------------------------------------------------------- surface integrals
 // kind 0: force on the faces of boundary type bc, F = -sum int stressVector ds
@@ -1542,19 +1390,32 @@ struct Launch {
         long long nt = (long long)M.nElem * NC;
         k_fd_col<Mdl, DIM, ORDER><<<(unsigned)((nt + kBlock - 1) / kBlock), kBlock, sm, s>>>(M, W, K0, KR0, h, a1, Adiag, Aneigh);
     }
+    // exact blocks and adjoint product: with the gradients' matrices where a model or the artificial
+    // viscosity reads gradients (the limiter leaves none without dampTol)
+    template <bool GRAD, int MODE, class T>
+    static void jacobian_as(const DevMesh& M, cudaStream_t s, const double* W, double a1, double* Ad, double* An, T* F,
+                            const double* lam, double* g) {
+        using C = JacCfg<Mdl, DIM, ORDER, GRAD>;
+        cudaFuncSetAttribute(k_jacobian<Mdl, DIM, ORDER, GRAD, MODE, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        k_jacobian<Mdl, DIM, ORDER, GRAD, MODE, T>
+            <<<(unsigned)((M.nElem + C::E - 1) / C::E), C::THREADS, C::SMEM, s>>>(M, W, a1, Ad, An, F, lam, g);
+    }
+    template <int MODE, class T>
+    static void jacobian(const DevMesh& M, cudaStream_t s, const double* W, double a1, double* Ad, double* An, T* F,
+                         const double* lam, double* g) {
+        if (Mdl::kViscous || Mdl::kSource || M.artificial)
+            jacobian_as<true, MODE, T>(M, s, W, a1, Ad, An, F, lam, g);
+        else if constexpr (!Mdl::kViscous && !Mdl::kSource)
+            jacobian_as<false, MODE, T>(M, s, W, a1, Ad, An, F, lam, g);
+    }
     static void jac_exact(const DevMesh& M, cudaStream_t s, const double* W, double a1, double* Adiag, double* Aneigh) {
-        constexpr int NC = Element<Mdl, DIM, ORDER>::NC;
-        long long nt = (long long)M.nElem * NC;
-        k_jac_exact<Mdl, DIM, ORDER><<<(unsigned)((nt + kBlock - 1) / kBlock), kBlock, 0, s>>>(M, W, a1, Adiag, Aneigh);
+        jacobian<JAC_BLOCKS, double>(M, s, W, a1, Adiag, Aneigh, nullptr, nullptr, nullptr);
     }
     static void jac_exact_factor(const DevMesh& M, cudaStream_t s, const double* W, double a1, void* F, int fp32) {
-        constexpr int NC = Element<Mdl, DIM, ORDER>::NC;
-        long long nt = (long long)M.nElem * NC;
-        const unsigned g = (unsigned)((nt + kBlock - 1) / kBlock);
         if (fp32)
-            k_jac_exact_factor<Mdl, DIM, ORDER, float><<<g, kBlock, 0, s>>>(M, W, a1, (float*)F);
+            jacobian<JAC_FACTOR, float>(M, s, W, a1, nullptr, nullptr, (float*)F, nullptr, nullptr);
         else
-            k_jac_exact_factor<Mdl, DIM, ORDER, double><<<g, kBlock, 0, s>>>(M, W, a1, (double*)F);
+            jacobian<JAC_FACTOR, double>(M, s, W, a1, nullptr, nullptr, (double*)F, nullptr, nullptr);
     }
     static void norms_elem(const DevMesh& M, cudaStream_t s, const double* R, double* out) {
         k_norms_elem<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, R, out);
@@ -1569,9 +1430,7 @@ struct Launch {
         k_gcl_mass<DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, a1, a2, a3, mass);
     }
     static void vjp(const DevMesh& M, cudaStream_t s, const double* W, const double* lam, double* g) {
-        constexpr int NC = Element<Mdl, DIM, ORDER>::NC;
-        long long nt = (long long)M.nElem * NC;
-        k_vjp_cols<Mdl, DIM, ORDER><<<(unsigned)((nt + kBlock - 1) / kBlock), kBlock, 0, s>>>(M, W, lam, g);
+        jacobian<JAC_VJP, double>(M, s, W, 0.0, nullptr, nullptr, nullptr, lam, g);
     }
     static void surface(const DevMesh& M, cudaStream_t s, const double* W, int kind, int bc, double* part, double* dIdW) {
         k_surface<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, 0, s>>>(M, W, kind, bc, part, dIdW);
