@@ -113,7 +113,7 @@ void free_all(fp_ctx* c) {
     c->h_scal = nullptr;
     if (c->h_part) cudaFreeHost(c->h_part);
     c->h_part = nullptr;
-    c->d_Adiag = c->d_Aneigh = c->d_rhs = c->d_K0 = c->d_KR0 = c->d_P64 = nullptr;
+    c->d_Adiag = c->d_Aneigh = c->d_rhs = c->d_KT = c->d_P64 = nullptr;
     c->d_mass = nullptr;
     c->d_vu = nullptr;
     c->n_cases = 0;
@@ -192,7 +192,7 @@ int ensure_implicit(fp_ctx* c) {
     if (c->d_Adiag) return FP_OK;
     const size_t ld = c->hm.ld, nc = c->nc, nf = c->hm.nf;
     if ((rc = dalloc(c, &c->d_Adiag, nc * nc * ld)) || (rc = dalloc(c, &c->d_Aneigh, nf * nc * nc * ld)) ||
-        (rc = dalloc(c, &c->d_K0, nc * ld)) || (rc = dalloc(c, &c->d_KR0, nf * nc * ld)))
+        (rc = dalloc(c, &c->d_KT, nf * nc * ld)))
         return rc;
     return FP_OK;
 }

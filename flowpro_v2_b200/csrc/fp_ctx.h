@@ -77,8 +77,7 @@ struct fp_ctx {
     double* d_Adiag = nullptr; // [nc*nc][ld]  untransposed: A[r][c] at (r*nc + c)*ld + e
     double* d_Aneigh = nullptr;// [nf][nc*nc][ld]
     double* d_rhs = nullptr;   // [nc][ld]
-    double* d_K0 = nullptr;    // FD base residual [nc][ld]
-    double* d_KR0 = nullptr;   // FD base face contributions [nf][nc][ld]
+    double* d_KT = nullptr;    // scratch of the transposed block product [nf][nc][ld]
     double* d_P64 = nullptr;   // inverse diagonal blocks, FP64 [nc*nc][ld]
     float* d_P32 = nullptr;    // inverse diagonal blocks, FP32
     int prec_ready = -1;       // precision of the factorised preconditioner, -1 none

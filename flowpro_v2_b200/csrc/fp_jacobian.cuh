@@ -1,5 +1,6 @@
-// Exact element Jacobian blocks and the adjoint product, from the flux Jacobians at the quadrature
-// points.  Column i = (mi, bi) of an element's blocks is the derivative of the element residual, and of the
+// Element Jacobian blocks: exact ones and the adjoint product here, finite differences below.
+//
+// Exact blocks come from the flux Jacobians at the quadrature points.  Column i = (mi, bi) of an element's blocks is the derivative of the element residual, and of the
 // element's face contributions to its neighbours, along the coefficient of basis function bi in equation
 // mi.  The integrand at a point depends on that coefficient through the state phi_bi and, where gradients
 // are read, the reference gradients dphi_bi, so the NE x NE matrices of the integrand with respect to the
@@ -357,6 +358,298 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
             for (int r = 0; r < NC; r++) Adiag[((size_t)r * NC + i) * ld + e] = K[r];
         } else {
             store_column<NC>(F + ((size_t)e * (1 + NF) * NC + i) * NC, K);
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------- finite differences
+// BDF2.assembleJacobiMatrix finite differences (BDF2.java:349-378): per element, the residual with
+// W + h e_i for every own unknown i; the diagonal block column A[r][i] = -(R_i[r] - R[r]) / h + a1 M, and
+// the block of each face neighbour A_nb[r][i] = (KR_i[r] - KR[r]) / h from this element's face integrals.
+//
+// Unlike the exact blocks every column needs the integrand itself at every point, and its digits: a rounding
+// of 1e-16 shows as 1e-8 in the difference, so every sum keeps the order of the element residual.
+//
+// A thread block takes E elements and all their columns together, the unperturbed one as column NC.  The
+// traces of all points are formed once (a thread per point, side and equation) and kept in shared memory;
+// a column replaces one equation's trace.  Per face, and per VCH volume points: a thread per element, point
+// and column evaluates the integrand into shared memory, then a thread per element, column and equation
+// (ITEMS of them, the NB sums in registers) adds it to its rows.
+//
+// What bounds it: the NC + 1 evaluations of the flux at each point.  A thread per element and column that
+// forms all traces itself, with 2 NC sums in local memory, measured, ms: 18,000 tetrahedra Euler p = 2
+// 8.4 -> 3.9; 50,416 triangles Navier-Stokes p = 2 3.1 -> 2.5.
+template <class Mdl, int DIM, int ORDER, bool GRAD>
+struct FdCfg {
+    using El = Element<Mdl, DIM, ORDER>;
+    static constexpr int NC = El::NC, NE = El::NE, NB = El::NB, COLS = NC + 1;
+    static constexpr int S = GRAD ? 1 + DIM : 1;
+    static constexpr bool VOLUME = ORDER > 1 || Mdl::kSource;
+    static constexpr int PF = El::NF * El::NQF, PV = VOLUME ? El::NQV : 0;
+    static constexpr int OUT = DIM + (Mdl::kSource ? 1 : 0);
+    static constexpr int cmax(int a, int b) { return a > b ? a : b; }
+    static constexpr int cmin(int a, int b) { return a < b ? a : b; }
+    static constexpr int VCH = cmin(El::NQV, cmax(2, El::NQF / OUT));  // volume points at a time
+    static constexpr int TRC = (2 * PF + PV) * NE * S;                 // traces: left and right of the faces, volume
+    static constexpr int INT = cmax(El::NQF * NE, VOLUME ? VCH * OUT * NE : 0) * COLS;
+    static constexpr int PER = NC + TRC + INT + NC;                    // coefficients, traces, integrands, base rows
+    static constexpr int THREADS = 256;
+    static constexpr int ITEMS_MAX = cmax(1, cmin(3, 24 / NB));
+    static constexpr int E = cmax(1, cmin(32, cmin(THREADS * ITEMS_MAX / (COLS * NE), (100 * 1024 / 8) / PER)));
+    static constexpr int ITEMS = (E * COLS * NE + THREADS - 1) / THREADS;
+    static constexpr size_t SMEM = (size_t)E * PER * sizeof(double);
+    static constexpr int CTAS = SMEM <= 112 * 1024 ? 2 : 1;
+};
+
+template <class Mdl, int DIM, int ORDER, bool GRAD>
+__global__ void __launch_bounds__(FdCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (FdCfg<Mdl, DIM, ORDER, GRAD>::CTAS))
+    k_fd(DevMesh M, const double* __restrict__ W, double h, double a1, double* __restrict__ Adiag, double* __restrict__ Aneigh) {
+    using C = FdCfg<Mdl, DIM, ORDER, GRAD>;
+    using El = Element<Mdl, DIM, ORDER>;
+    using TB = Tab<DIM, ORDER>;
+    using GL = GeoLayout<DIM>;
+    constexpr int NC = C::NC, NE = C::NE, NB = C::NB, NF = El::NF, NQF = El::NQF, NQV = El::NQV, NP = El::NP, S = C::S, E = C::E;
+    constexpr int COLS = C::COLS, SLOT = E * COLS, NG = GRAD ? DIM * NE : 1;
+    extern __shared__ __align__(16) double fp_dyn_smem[];
+    double* coef = fp_dyn_smem;           // [c][element]
+    double* trc = coef + E * NC;          // [point and side][equation][value, gradient][element]
+    double* gw = trc + E * C::TRC;        // [point][component][column][element]
+    double* base = gw + E * C::INT;       // [row][element] of the unperturbed column
+    const int e0 = blockIdx.x * E, n = min(E, M.nElem - e0);
+    const int ld = M.ld;
+
+    for (int t = threadIdx.x; t < NC * E; t += C::THREADS) {
+        const int x = t % E;
+        coef[t] = x < n ? ldg(W + (size_t)(t / E) * ld + e0 + x) : 0.0;
+    }
+    __syncthreads();
+    // ------------------------------------------------------------------ traces
+    for (int t = threadIdx.x; t < (2 * C::PF + C::PV) * NE * E; t += C::THREADS) {
+        const int x = t % E, y = t / E, m = y % NE, pt = y / NE, e = e0 + x;
+        if (x >= n) continue;
+        const double *phi, *dphi;
+        int eo = e;  // the element the trace is of
+        bool own = true;
+        if (pt < C::PF) {
+            phi = M.tab + TB::o_phiL + pt * NB;
+            dphi = M.tab + TB::o_dphiL + pt * NB * DIM;
+        } else if (pt < 2 * C::PF) {
+            const int q = pt - C::PF, k = q / NQF, p = q - k * NQF;
+            eo = M.tt[(size_t)k * ld + e];
+            if (eo < 0) continue;
+            own = false;
+            const int fc = M.fcode[(size_t)k * ld + e];
+            phi = M.tab + TB::o_phiR + (fc * NQF + p) * NB;
+            dphi = M.tab + TB::o_dphiR + (fc * NQF + p) * NB * DIM;
+        } else {
+            phi = M.tab + TB::o_phi + (pt - 2 * C::PF) * NB;
+            dphi = M.tab + TB::o_dphi + (pt - 2 * C::PF) * NB * DIM;
+        }
+        double v, gr[DIM], dv[DIM];
+        El::template trace_sums<GRAD>(
+            phi, dphi, [&](int j) { return own ? coef[(m * NB + j) * E + x] : ldg(W + (size_t)(m * NB + j) * ld + eo); }, v, gr, 1);
+        double* o = trc + (size_t)(y * S) * E + x;
+        o[0] = v;
+        if constexpr (GRAD) {
+            double Ji[DIM * DIM];
+#pragma unroll
+            for (int c = 0; c < DIM * DIM; c++) Ji[c] = ldg(M.geo + (size_t)(GL::JINV + c) * ld + eo);
+            El::physical_gradient(Ji, gr, dv, 1);
+#pragma unroll
+            for (int d = 0; d < DIM; d++) o[(1 + d) * E] = dv[d];
+        }
+    }
+    // the traces of a point with column i's perturbation: equation mi's is formed again
+    auto perturbed = [&](int pt, int x, int i, const double* phi, const double* dphi, const double* Ji, double* v, double* dv) {
+        const int mi = i / NB, bi = i - mi * NB;
+        double pv = 0.0, pg[DIM], pd[DIM];
+        if (i < NC) {
+            El::template trace_sums<GRAD>(
+                phi, dphi,
+                [&](int j) {
+                    const double c = coef[(mi * NB + j) * E + x];
+                    return j == bi ? c + h : c;
+                },
+                pv, pg, 1);
+            if constexpr (GRAD) El::physical_gradient(Ji, pg, pd, 1);
+        }
+        const double* o = trc + (size_t)(pt * NE * S) * E + x;
+#pragma unroll
+        for (int m = 0; m < NE; m++) {
+            v[m] = m == mi ? pv : o[m * S * E];
+            if constexpr (GRAD) {
+#pragma unroll
+                for (int d = 0; d < DIM; d++) dv[d * NE + m] = m == mi ? pd[d] : o[(m * S + 1 + d) * E];
+            }
+        }
+    };
+    double K[C::ITEMS][NB];
+#pragma unroll
+    for (int u = 0; u < C::ITEMS; u++)
+#pragma unroll
+        for (int j = 0; j < NB; j++) K[u][j] = 0.0;
+    const double invh = 1.0 / h;
+    // ------------------------------------------------------------------ faces
+#pragma unroll 1
+    for (int k = 0; k < NF; k++) {
+        __syncthreads();  // traces; integrands of the last face read
+        for (int t = threadIdx.x; t < NQF * SLOT; t += C::THREADS) {
+            const int x = t % E, y = t / E, i = y % COLS, p = y / COLS, pt = k * NQF + p, e = e0 + x;
+            if (x >= n) continue;
+            const int TT = M.tt[(size_t)k * ld + e];
+            const bool interior = TT > -1;
+            double Ji[GRAD ? DIM * DIM : 1], WL[NE], WR[NE], dWL[NG], dWR[NG], Cc[NE], Jm[NE];
+            if constexpr (GRAD) {
+#pragma unroll
+                for (int c = 0; c < DIM * DIM; c++) Ji[c] = ldg(M.geo + (size_t)(GL::JINV + c) * ld + e);
+            }
+            perturbed(pt, x, i, M.tab + TB::o_phiL + pt * NB, M.tab + TB::o_dphiL + pt * NB * DIM, Ji, WL, dWL);
+            if (interior) {
+                const double* o = trc + (size_t)((C::PF + pt) * NE * S) * E + x;
+#pragma unroll
+                for (int m = 0; m < NE; m++) {
+                    WR[m] = o[m * S * E];
+                    if constexpr (GRAD) {
+#pragma unroll
+                        for (int d = 0; d < DIM; d++) dWR[d * NE + m] = o[(m * S + 1 + d) * E];
+                    }
+                }
+            }
+            double nrm[DIM], Jac, dL;
+            El::face_geo(M, e, k, nrm, Jac, dL);
+            El::template point_flux<GRAD>(M, e, k, p, TT, nrm, dL, ldg(M.eps + e), interior ? ldg(M.eps + TT) : 0.0, WL, WR, dWL,
+                                          dWR, Cc, Jm);
+            const double jw = Jac * ldg(M.tab + TB::o_wf + p);
+            const bool ip = Mdl::kViscous && (interior || Mdl::isIPFace(TT));
+            const double cip = ip ? ldg(M.cip + e) : 0.0;
+            double* o = gw + (size_t)p * NE * SLOT + i * E + x;
+#pragma unroll
+            for (int m = 0; m < NE; m++) {
+                double g = Cc[m];
+                if (ip) g -= cip * Jm[m];
+                o[m * SLOT] = jw * g;
+            }
+        }
+        __syncthreads();
+        double acc[C::ITEMS][NB];
+#pragma unroll
+        for (int u = 0; u < C::ITEMS; u++) {
+            const int t = threadIdx.x + u * C::THREADS, s = t % SLOT, m = t / SLOT, x = s % E;
+            if (m >= NE || x >= n) continue;
+            const int nb = M.tt[(size_t)k * ld + e0 + x];
+            const int fc = nb > -1 ? M.fcode[(size_t)k * ld + e0 + x] : 0;
+            const double* phiL = M.tab + TB::o_phiL + k * NQF * NB;
+            const double* phiR = M.tab + TB::o_phiR + fc * NQF * NB;
+#pragma unroll
+            for (int j = 0; j < NB; j++) acc[u][j] = 0.0;
+#pragma unroll 1
+            for (int p = 0; p < NQF; p++) {
+                const double g = gw[(p * NE + m) * SLOT + s];
+#pragma unroll
+                for (int j = 0; j < NB; j++) {
+                    K[u][j] += g * ldg(phiL + p * NB + j);
+                    acc[u][j] += g * ldg(phiR + p * NB + j);
+                }
+            }
+            if (s / E == NC) {
+#pragma unroll
+                for (int j = 0; j < NB; j++) base[(m * NB + j) * E + x] = acc[u][j];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < C::ITEMS; u++) {
+            const int t = threadIdx.x + u * C::THREADS, s = t % SLOT, m = t / SLOT, x = s % E, i = s / E;
+            if (m >= NE || x >= n || i == NC) continue;
+            const int nb = M.tt[(size_t)k * ld + e0 + x];
+            if (nb < 0) continue;
+            // block of element nb for its face kr, column i (this element's unknown i)
+            const int kr = M.fcode[(size_t)k * ld + e0 + x] / NP;
+            double* A = Aneigh + (size_t)kr * NC * NC * ld;
+#pragma unroll
+            for (int j = 0; j < NB; j++)
+                A[((size_t)(m * NB + j) * NC + i) * ld + nb] = (acc[u][j] - base[(m * NB + j) * E + x]) * invh;
+        }
+    }
+    // ------------------------------------------------------------------ volume
+    if constexpr (C::VOLUME) {
+#pragma unroll 1
+        for (int q0 = 0; q0 < NQV; q0 += C::VCH) {
+            const int nq = min(C::VCH, NQV - q0);
+            __syncthreads();  // integrands of the last points read
+            for (int t = threadIdx.x; t < nq * SLOT; t += C::THREADS) {
+                const int x = t % E, y = t / E, i = y % COLS, r = y / COLS, q = q0 + r, e = e0 + x;
+                if (x >= n) continue;
+                double Ji[DIM * DIM], WI[NE], dWI[DIM * NE], Gr[DIM * NE], sw[NE];
+#pragma unroll
+                for (int c = 0; c < DIM * DIM; c++) Ji[c] = ldg(M.geo + (size_t)(GL::JINV + c) * ld + e);
+                perturbed(2 * C::PF + q, x, i, M.tab + TB::o_phi + q * NB, M.tab + TB::o_dphi + q * NB * DIM, Ji, WI, dWI);
+                if constexpr (!GRAD) {  // nothing reads the gradient: its coefficient is exactly zero
+#pragma unroll
+                    for (int c = 0; c < DIM * NE; c++) dWI[c] = 0.0;
+                }
+                const double jac = ldg(M.geo + (size_t)GL::JAC * ld + e);
+                El::volume_point(M, e, q, Ji, jac * ldg(M.tab + TB::o_w + q), ldg(M.eps + e) + M.dampConst, WI, dWI, Gr, sw);
+                double* o = gw + (size_t)r * C::OUT * NE * SLOT + i * E + x;
+                if constexpr (ORDER > 1) {
+#pragma unroll
+                    for (int c = 0; c < DIM * NE; c++) o[c * SLOT] = Gr[c];
+                }
+                if constexpr (Mdl::kSource) {
+#pragma unroll
+                    for (int m = 0; m < NE; m++) o[(DIM * NE + m) * SLOT] = sw[m];
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < C::ITEMS; u++) {
+                const int t = threadIdx.x + u * C::THREADS, s = t % SLOT, m = t / SLOT;
+                if (m >= NE || s % E >= n) continue;
+#pragma unroll 1
+                for (int r = 0; r < nq; r++) {
+                    const double *phi = M.tab + TB::o_phi + (q0 + r) * NB, *dphi = M.tab + TB::o_dphi + (q0 + r) * NB * DIM;
+                    const double* o = gw + (size_t)(r * C::OUT * NE + m) * SLOT + s;
+                    if constexpr (ORDER > 1) {
+                        double gd[DIM];
+#pragma unroll
+                        for (int d = 0; d < DIM; d++) gd[d] = o[d * NE * SLOT];
+#pragma unroll
+                        for (int j = 0; j < NB; j++)
+#pragma unroll
+                            for (int d = 0; d < DIM; d++) K[u][j] += gd[d] * ldg(dphi + j * DIM + d);
+                    }
+                    if constexpr (Mdl::kSource) {
+                        const double sm = o[DIM * NE * SLOT];
+#pragma unroll
+                        for (int j = 0; j < NB; j++) K[u][j] += sm * ldg(phi + j);
+                    }
+                }
+            }
+        }
+    }
+    // ------------------------------------------------------------------ diagonal block
+    __syncthreads();  // the last face's base rows have been read
+#pragma unroll
+    for (int u = 0; u < C::ITEMS; u++) {
+        const int t = threadIdx.x + u * C::THREADS, s = t % SLOT, m = t / SLOT, x = s % E;
+        if (m >= NE || x >= n || s / E != NC) continue;
+#pragma unroll
+        for (int j = 0; j < NB; j++) base[(m * NB + j) * E + x] = K[u][j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < C::ITEMS; u++) {
+        const int t = threadIdx.x + u * C::THREADS, s = t % SLOT, m = t / SLOT, x = s % E, i = s / E;
+        if (m >= NE || x >= n || i == NC) continue;
+        const int e = e0 + x, mi = i / NB, bi = i - mi * NB;
+        double c1 = a1;
+        case_coefficients(M, e, c1);
+        const double jac = ldg(M.geo + (size_t)GL::JAC * ld + e);
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+            double a = (K[u][j] - base[(m * NB + j) * E + x]) / (-h);
+            if (m == mi) a += c1 * mass_entry<DIM, ORDER>(M, e, 0, j, bi, jac);
+            Adiag[((size_t)(m * NB + j) * NC + i) * ld + e] = a;
         }
     }
 }

@@ -117,15 +117,6 @@ struct NbDual {
     }
 };
 
-struct NoKR {
-    static constexpr bool enabled = false;
-    template <class T>
-    __device__ void begin(int) {}
-    template <class T>
-    __device__ void add(int, int, const T&) {}
-    __device__ void end(int, int, int) {}
-};
-
 template <class Mdl, int DIM, int ORDER>
 struct Element {
     using TB = Tab<DIM, ORDER>;
@@ -173,32 +164,42 @@ struct Element {
         constexpr int NG = GRAD ? DIM * NE : 1;
         T g[NG];
 #pragma unroll
-        for (int m = 0; m < NE; m++) {
-            W[m] = 0.0;
-            if constexpr (GRAD) {
-#pragma unroll
-                for (int d = 0; d < DIM; d++) g[d * NE + m] = 0.0;
-            }
-#pragma unroll
-            for (int j = 0; j < NB; j++) {
-                const T c = coef(m * NB + j);
-                W[m] += c * ldg(phi + j);
-                if constexpr (GRAD) {
-#pragma unroll
-                    for (int d = 0; d < DIM; d++) g[d * NE + m] += c * ldg(dphi + j * DIM + d);
-                }
-            }
-        }
+        for (int m = 0; m < NE; m++)
+            trace_sums<GRAD>(phi, dphi, [&](int j) { return coef(m * NB + j); }, W[m], GRAD ? g + m : g, NE);
         if constexpr (GRAD) {
 #pragma unroll
-            for (int m = 0; m < NE; m++)
+            for (int m = 0; m < NE; m++) physical_gradient(Ji, g + m, dW + m, NE);
+        }
+    }
+
+    // one equation's value and (GRAD) reference gradient g[d * stride], coefficients coef(j)
+    template <bool GRAD, class T, class Coef>
+    static __device__ __forceinline__ void trace_sums(const double* phi, const double* dphi, const Coef& coef, T& W, T* g, int stride) {
+        W = 0.0;
+        if constexpr (GRAD) {
 #pragma unroll
-                for (int d = 0; d < DIM; d++) {
-                    T s = 0.0;
+            for (int d = 0; d < DIM; d++) g[d * stride] = 0.0;
+        }
 #pragma unroll
-                    for (int q = 0; q < DIM; q++) s += Ji[q * DIM + d] * g[q * NE + m];
-                    dW[d * NE + m] = s;
-                }
+        for (int j = 0; j < NB; j++) {
+            const T c = coef(j);
+            W += c * ldg(phi + j);
+            if constexpr (GRAD) {
+#pragma unroll
+                for (int d = 0; d < DIM; d++) g[d * stride] += c * ldg(dphi + j * DIM + d);
+            }
+        }
+    }
+
+    // an equation's physical gradient dW[d * stride] from the reference gradient g[d * stride]
+    template <class T>
+    static __device__ __forceinline__ void physical_gradient(const double* Ji, const T* g, T* dW, int stride) {
+#pragma unroll
+        for (int d = 0; d < DIM; d++) {
+            T s = 0.0;
+#pragma unroll
+            for (int q = 0; q < DIM; q++) s += Ji[q * DIM + d] * g[q * stride];
+            dW[d * stride] = s;
         }
     }
 
@@ -311,11 +312,10 @@ struct Element {
     }
 
     // DGpure.residuum (faces then volume), element e, own coefficients w (already W + V).
-    // nbl(c, nb) returns the coefficients of a neighbour; kr receives the contribution of
-    // this element's face integrals to the neighbour's residual (DGpure.residuumWall's KR).
+    // nbl(c, nb) returns the coefficients of a neighbour.
     // w: a register array or an accessor reading the coefficients from memory
-    template <class T, class WA, class NbL, class KR>
-    static __device__ void residual(const DevMesh& M, int e, const WA& w, const NbL& nbl, T* K, KR& kr) {
+    template <class T, class WA, class NbL>
+    static __device__ void residual(const DevMesh& M, int e, const WA& w, const NbL& nbl, T* K) {
         const int ld = M.ld;
         double Jinv[DIM * DIM];
 #pragma unroll
@@ -343,7 +343,6 @@ struct Element {
             }
             const bool ip = Mdl::kViscous && (interior || Mdl::isIPFace(TT));
             const bool grads = needs_gradients(M, interior, eps_e, eps_nb);
-            if (KR::enabled && interior) kr.template begin<T>(k);
 #pragma unroll 1
             for (int p = 0; p < NQF; p++) {
                 T C[NE], Jm[NE];
@@ -364,14 +363,8 @@ struct Element {
                     const T gw = jw * g;
 #pragma unroll
                     for (int j = 0; j < NB; j++) K[m * NB + j] += gw * ldg(phiL + j);
-                    if (KR::enabled && interior) {
-                        const double* phiR = M.tab + TB::o_phiR + ((kr_face * NP + pm) * NQF + p) * NB;
-#pragma unroll
-                        for (int j = 0; j < NB; j++) kr.add(k, m * NB + j, gw * ldg(phiR + j));
-                    }
                 }
             }
-            if (KR::enabled && interior) kr.end(k, TT, kr_face);
         }
         volume(M, e, w, Jinv, eps_e, K);
     }

@@ -45,8 +45,7 @@ struct Launchers {
     void (*dtbound)(const DevMesh&, cudaStream_t, const double* W, double factor, double* part) = nullptr;
     void (*rhs)(const DevMesh&, cudaStream_t, const double* W, const double* Wo, const double* Wo2, double a1, double a2,
                 double a3, double* R, double* rhs, double* part) = nullptr;
-    void (*fd)(const DevMesh&, cudaStream_t, const double* W, double* K0, double* KR0, double h, double a1, double* Adiag,
-               double* Aneigh) = nullptr;
+    void (*fd)(const DevMesh&, cudaStream_t, const double* W, double h, double a1, double* Adiag, double* Aneigh) = nullptr;
     void (*jac_exact)(const DevMesh&, cudaStream_t, const double* W, double a1, double* Adiag, double* Aneigh) = nullptr;
     // exact blocks into the block ILU(0) factor storage (float when fp32, else double)
     void (*jac_exact_factor)(const DevMesh&, cudaStream_t, const double* W, double a1, void* F, int fp32) = nullptr;

@@ -436,7 +436,7 @@ int mass_shift(fp_ctx* c, double delta) {
 int spmv_t(fp_ctx* c, const double* x, double* y) {
     const int nE = c->hm.nElem;
     const dim3 g(c->nc, (nE + 127) / 128), g3(c->nc, (nE + 127) / 128, 1 + c->hm.nf);
-    double* Z = c->d_KR0;  // scratch of the finite-difference assembly, allocated with the blocks
+    double* Z = c->d_KT;
     k_spmv_t_own<<<g3, 128, 0, c->stream>>>(nE, c->hm.ld, c->nc, c->d_Adiag, c->d_Aneigh, c->d_tt, x, y, Z);
     k_spmv_t_gather<<<g, 128, 0, c->stream>>>(nE, c->hm.ld, c->nc, c->hm.nf, c->hm.tab.nperm, c->d_tt, c->d_fcode, Z, y);
     return cuda_check(c, cudaGetLastError(), "spmv_t");

@@ -405,7 +405,7 @@ int launch_fd_jacobian(fp_ctx* c, double a1, double a2, double a3, double* rhs_n
     const Launchers* t = L(c, rc);
     if (!t) return rc;
     prof_begin(c, PH_BLOCKS);
-    t->fd(dev_mesh(c), c->stream, c->d_W, c->d_K0, c->d_KR0, c->hm.num.fd_step, a1, c->d_Adiag, c->d_Aneigh);
+    t->fd(dev_mesh(c), c->stream, c->d_W, c->hm.num.fd_step, a1, c->d_Adiag, c->d_Aneigh);
     prof_end(c);
     return cuda_check(c, cudaGetLastError(), "fd jacobian");
 }

@@ -89,22 +89,6 @@ struct OwnDualShared {
         return x;
     }
 };
-// the finite-difference kernels' coefficients, [c][thread], in dynamic shared memory
-template <int NC>
-constexpr size_t fd_smem_bytes() {
-    return (size_t)NC * kBlock * sizeof(double);
-}
-// coefficient c of W + V with V = h e_i (the perturbed column of the finite-difference Jacobian)
-template <int BLOCK>
-struct OwnPerturbed {
-    const double* p;
-    int i;
-    double h;
-    __device__ double operator[](int c) const {
-        const double v = p[c * BLOCK];
-        return c == i ? v + h : v;
-    }
-};
 #define FP_OWN_COEFFS(NC_)                                                   \
     __shared__ double own_wsh_static[(NC_) <= kShNC ? (NC_) * kBlock : 1]; \
     double* own_wsh = (NC_) <= kShNC ? own_wsh_static : fp_dyn_smem
@@ -409,8 +393,7 @@ __global__ void __launch_bounds__(kBlock)
     else
         w = wr;
     Dual<1> K[NC];
-    NoKR kr;
-    El::residual(M, e, w, NbDual<1>{W, V, ld}, K, kr);
+    El::residual(M, e, w, NbDual<1>{W, V, ld}, K);
     const double jac = ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
 #pragma unroll
     for (int m = 0; m < NE; m++)
@@ -941,110 +924,6 @@ __global__ void __launch_bounds__(kBlock, (MinBlocks<Mdl, DIM, ORDER>::elem))
     if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
-// ---------------------------------------------------------------------------- FD Jacobian
-// BDF2.assembleJacobiMatrix finite differences (BDF2.java:349-378): per element, the
-// residual with W + h e_i for every own unknown i; the diagonal block column
-// A[r][i] = -(R_i[r] - R[r]) / h + a1 M, and the block of each face neighbour
-// A_nb[r][i] = (KR_i[r] - KR[r]) / h from this element's face integrals.
-template <int NC>
-struct KRBase {
-    static constexpr bool enabled = true;
-    double acc[NC];
-    double* KR0;
-    int ld, e;
-    template <class T>
-    __device__ void begin(int) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) acc[c] = 0;
-    }
-    __device__ void add(int, int c, double v) { acc[c] += v; }
-    __device__ void end(int k, int, int) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) KR0[((size_t)k * NC + c) * ld + e] = acc[c];
-    }
-};
-
-template <int NC>
-struct KRCol {
-    static constexpr bool enabled = true;
-    double acc[NC];
-    const double* KR0;
-    double* Aneigh;
-    int ld, e, i;
-    double invh;
-    template <class T>
-    __device__ void begin(int) {
-#pragma unroll
-        for (int c = 0; c < NC; c++) acc[c] = 0;
-    }
-    __device__ void add(int, int c, double v) { acc[c] += v; }
-    __device__ void end(int k, int nb, int kr) {
-        // block of element nb for its face kr, column i (this element's unknown i)
-        double* A = Aneigh + (size_t)kr * NC * NC * ld;
-#pragma unroll
-        for (int r = 0; r < NC; r++)
-            A[((size_t)r * NC + i) * ld + nb] = (acc[r] - ldg(KR0 + ((size_t)k * NC + r) * ld + e)) * invh;
-    }
-};
-
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_fd_base(DevMesh M, const double* __restrict__ W, double* __restrict__ K0, double* __restrict__ KR0) {
-    using El = E<Mdl, DIM, ORDER>;
-    constexpr int NC = El::NC;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= M.nElem) return;
-    double* wsh = fp_dyn_smem;
-#pragma unroll
-    for (int c = 0; c < NC; c++) wsh[c * kBlock + threadIdx.x] = ldg(W + (size_t)c * M.ld + e);
-    const OwnShared<kBlock> w{wsh + threadIdx.x};
-    double K[NC];
-    KRBase<NC> kr;
-    kr.KR0 = KR0;
-    kr.ld = M.ld;
-    kr.e = e;
-    El::residual(M, e, w, NbPlain{W, M.ld}, K, kr);
-#pragma unroll
-    for (int c = 0; c < NC; c++) K0[(size_t)c * M.ld + e] = K[c];
-}
-
-template <class Mdl, int DIM, int ORDER>
-__global__ void __launch_bounds__(kBlock)
-    k_fd_col(DevMesh M, const double* __restrict__ W, const double* __restrict__ K0, const double* __restrict__ KR0, double h,
-             double a1, double* __restrict__ Adiag, double* __restrict__ Aneigh) {
-    using El = E<Mdl, DIM, ORDER>;
-    using TB = Tab<DIM, ORDER>;
-    constexpr int NC = El::NC, NB = El::NB;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const int e = (int)(t % M.nElem);
-    const int i = (int)(t / M.nElem);
-    if (i >= NC) return;
-    case_coefficients(M, e, a1);
-    const int ld = M.ld;
-    double* wsh = fp_dyn_smem;
-#pragma unroll
-    for (int c = 0; c < NC; c++) wsh[c * kBlock + threadIdx.x] = ldg(W + (size_t)c * ld + e);
-    const OwnPerturbed<kBlock> w{wsh + threadIdx.x, i, h};  // W + V with V[i] = h (DGpure.residuum)
-    double K[NC];
-    KRCol<NC> kr;
-    kr.KR0 = KR0;
-    kr.Aneigh = Aneigh;
-    kr.ld = ld;
-    kr.e = e;
-    kr.i = i;
-    kr.invh = 1.0 / h;
-    El::residual(M, e, w, NbPlain{W, ld}, K, kr);
-    const double jac = ldg(M.geo + (size_t)GeoLayout<DIM>::JAC * ld + e);
-    const int mi = i / NB, bi = i - mi * NB;
-#pragma unroll
-    for (int r = 0; r < NC; r++) {
-        double a = (K[r] - ldg(K0 + (size_t)r * ld + e)) / (-h);
-        const int mr = r / NB, br = r - mr * NB;
-        if (mr == mi) a += a1 * mass_entry<DIM, ORDER>(M, e, 0, br, bi, jac);
-        Adiag[((size_t)r * NC + i) * ld + e] = a;
-    }
-}
-
 // ---------------------------------------------------------------------------- moving mesh
 // Mass matrix of time level lev from the current geometry (DGpure.recalculateMassMatrix,
 // DGpure.java:575-593): M_ij = sum_p jac w_p phi_i(p) phi_j(p), in the reference's order.
@@ -1312,11 +1191,6 @@ struct Launch {
             cudaFuncSetAttribute(k_face_tan<Mdl, DIM, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mf);
             cudaFuncSetAttribute(k_matfree_elem<Mdl, DIM, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mf);
         }
-        constexpr size_t fd = fd_smem_bytes<Element<Mdl, DIM, ORDER>::NC>();
-        if (fd > 48 * 1024) {
-            cudaFuncSetAttribute(k_fd_base<Mdl, DIM, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd);
-            cudaFuncSetAttribute(k_fd_col<Mdl, DIM, ORDER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fd);
-        }
         done.fetch_or(bit, std::memory_order_release);
     }
     static void faces(const DevMesh& M, cudaStream_t s, const double* W) {
@@ -1381,14 +1255,19 @@ struct Launch {
         faces(M, s, W);
         k_rhs<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, kDyn, s>>>(M, W, Wo, Wo2, a1, a2, a3, R, rhs, part);
     }
-    static void fd(const DevMesh& M, cudaStream_t s, const double* W, double* K0, double* KR0, double h, double a1,
-                   double* Adiag, double* Aneigh) {
-        constexpr int NC = Element<Mdl, DIM, ORDER>::NC;
-        prepare();
-        constexpr size_t sm = fd_smem_bytes<NC>();
-        k_fd_base<Mdl, DIM, ORDER><<<grid_of(M.nElem), kBlock, sm, s>>>(M, W, K0, KR0);
-        long long nt = (long long)M.nElem * NC;
-        k_fd_col<Mdl, DIM, ORDER><<<(unsigned)((nt + kBlock - 1) / kBlock), kBlock, sm, s>>>(M, W, K0, KR0, h, a1, Adiag, Aneigh);
+    // finite-difference blocks, with the traces' gradients where they are read, as below
+    template <bool GRAD>
+    static void fd_as(const DevMesh& M, cudaStream_t s, const double* W, double h, double a1, double* Adiag, double* Aneigh) {
+        using C = FdCfg<Mdl, DIM, ORDER, GRAD>;
+        cudaFuncSetAttribute(k_fd<Mdl, DIM, ORDER, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+        k_fd<Mdl, DIM, ORDER, GRAD>
+            <<<(unsigned)((M.nElem + C::E - 1) / C::E), C::THREADS, C::SMEM, s>>>(M, W, h, a1, Adiag, Aneigh);
+    }
+    static void fd(const DevMesh& M, cudaStream_t s, const double* W, double h, double a1, double* Adiag, double* Aneigh) {
+        if (Mdl::kViscous || Mdl::kSource || M.artificial)
+            fd_as<true>(M, s, W, h, a1, Adiag, Aneigh);
+        else if constexpr (!Mdl::kViscous && !Mdl::kSource)
+            fd_as<false>(M, s, W, h, a1, Adiag, Aneigh);
     }
     // exact blocks and adjoint product: with the gradients' matrices where a model or the artificial
     // viscosity reads gradients (the limiter leaves none without dampTol)

@@ -64,3 +64,42 @@ def test_blocks_and_adjoint_product_match_the_tangent(kind, order, damp):
     assert np.max(np.abs(Av + jv)) <= 1e-11 * np.max(np.abs(jv))
     assert np.max(np.abs(At + jl)) <= 1e-11 * np.max(np.abs(jl))
     g.close()
+
+
+@pytest.mark.parametrize("kind,order,damp", CASES)
+def test_finite_difference_blocks_match_differences_of_the_residual(kind, order, damp):
+    """A column of the finite-difference blocks against the difference of two residuals of the whole mesh
+    (the face and element passes).  Both round sums of a few dozen terms of the size |A| |W|, and the
+    difference is divided by h: 64 x 2^-52 / h = 1.4e-6 of that size."""
+    props = MODELS[kind][0](order)
+    wall = meshgen.WALL if kind in ("ns", "sa", "ns3") else meshgen.INVISCID_WALL
+    if damp:
+        props["dampTol"] = 3.0
+    m, tt = cases.channel(7, 5, seed=order, wall=wall) if MODELS[kind][1] == "channel" else cases.box(3, 2, 2, seed=2, wall=wall)
+    if kind == "sa":
+        m.wall_distance[:] = np.maximum(m.wall_distance, 1e-3)
+    g = fg.GpuMesh(props, m.vertices, m.elements, tt, m.wall_distance)
+    rng = np.random.default_rng(order)
+    w0 = g.get_state(0)
+    W = cases.perturbed(w0, g.n_basis, g.n_eqs, rng, 0.1 if damp else 0.02) if np.any(w0) else 0.1 * rng.standard_normal(w0.shape)
+    for which in (0, 1, 2):
+        g.set_state(W, which)
+    g.limiter()
+    asm = fg.JacobiAssembler(g, bdf_order=1)
+    asm.assemble(0.0, -1)  # no mass term
+    diag, neigh, _ = asm.blocks()
+    h = 1e-8
+    tol = 64 * 2.0 ** -52 / h * max(np.max(np.abs(diag)), np.max(np.abs(neigh))) * max(1.0, np.max(np.abs(W)))
+    R = g.residuum(W)
+    last = len(tt) - 1  # the last element: its block is partly empty
+    for e, i in [(0, 0), (last, W.shape[1] - 1)] + [(int(rng.integers(len(tt))), int(rng.integers(W.shape[1]))) for _ in range(4)]:
+        Wp = W.copy()
+        Wp[e, i] += h
+        d = (g.residuum(Wp) - R) / h
+        want = np.zeros_like(d)
+        want[e] = -diag[e, i]
+        for k in range(tt.shape[1]):  # neighbours whose face k is e's
+            for f in np.nonzero(tt[:, k] == e)[0]:
+                want[f] -= neigh[f, k, i]
+        assert np.max(np.abs(d - want)) <= tol
+    g.close()
