@@ -178,9 +178,9 @@ int fp_residual_timed(fp_ctx* ctx, int n, double* ms_face, double* ms_elem);
 int fp_jvp(fp_ctx* ctx, const double* v, double* dr);
 /* Adjoint of the residual: g = (dR/dW)^T lambda at the resident state (replaces the product
  * with the transposed assembled Jacobian that OptimisationToolExport writes,
- * OptimisationToolExport.java:38-260).  No Jacobian is stored: each element column is formed
- * in registers by the exact tangent of the element residual (quadrature states recomputed) and
- * contracted with lambda at once; stored blocks, if any, are left as they are. */
+ * OptimisationToolExport.java:38-260).  No Jacobian is stored: the exact
+ * tangents of the integrands at the quadrature points are contracted with lambda at once; stored
+ * blocks, if any, are left as they are. */
 int fp_vjp(fp_ctx* ctx, const double* lambda, double* g);
 /* Positivity limiter (Element.positivityLimiter, Element.java:385-476); returns #limited in *n. */
 int fp_positivity_limiter(fp_ctx* ctx, int* n_limited);
