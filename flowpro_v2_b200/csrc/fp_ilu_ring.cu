@@ -35,12 +35,12 @@
 #include <type_traits>
 
 #include "fp_ctx.h"
+#include "fp_ring_rule.h"
 
 namespace fp {
 
 namespace {
 
-constexpr int kRing = 64;      // positions a thread block may have between request and release
 constexpr int kMaxBlocks = 128;  // blocks of the ring
 constexpr int kFaces = 4;
 constexpr unsigned long long kEmpty = ~0ull;  // an unpublished word: a NaN no arithmetic produces
@@ -68,6 +68,7 @@ struct Cfg {
     static constexpr int WC = GPW * CW;                          // columns of a warp
     static constexpr int WARPS = 16;                             // consumer warps (one more is the producer)
     static constexpr int GROUPS = WARPS / WG;                    // elements in flight per thread block
+    static_assert(GROUPS <= kRingSlots / 2, "the producer keeps at least as many positions ahead as are in work");
     static constexpr int ROUNDS = ((FPW + 1) * WC + 31) / 32;    // words a lane fetches
     static constexpr int WV = (FPW + 2) * WC;                    // a warp's values: faces, own, before inv(U_ii)
     static constexpr int PART = 2 * P * NC;                      // partial sums of an element, two buffers
@@ -204,16 +205,18 @@ __device__ __forceinline__ void group_sync(int grp) {
 // order, requests their blocks in that order and releases them in bounded time, and all thread
 // blocks are co-resident (cooperative launch), so each wait ends; each is bounded all the same.
 // A wait for a value that gives up sets FP_DEV_TIMEOUT and the abort word, which ends every other
-// one; the sweep then runs to its end with garbage.  A wait for a copy that gives up (a bulk copy
-// lands within microseconds) also ends this thread block's loops.
+// one; the sweep then runs to its end with garbage.  The waits on the ring's barriers (kBarPolls: for
+// blocks on their way, and the producer's for a position to be released, which includes that
+// position's waits for values) do the same and set `dead`: the producer requests nothing more, and
+// the consumers pass the remaining positions without reading blocks that were not requested for them.
 template <class T, int NC>
 __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS) k_sweep_ring(SweepArgs A, const T* __restrict__ F) {
     using C = Cfg<T, NC>;
     constexpr int NC2 = NC * NC;
     extern __shared__ __align__(128) unsigned char ring_smem[];
-    __shared__ __align__(8) unsigned long long full[kRing], empty[kRing];
-    __shared__ int first[kRing];
-    __shared__ int cnts[kRing];  // producer's own: blocks of each position
+    __shared__ __align__(8) unsigned long long full[kRingSlots], empty[kRingSlots];
+    __shared__ int first[kRingSlots];
+    __shared__ int cnts[kRingSlots];  // producer's own: blocks of each position
     __shared__ volatile int dead;
     T* ring = reinterpret_cast<T*>(ring_smem);
     double* work = reinterpret_cast<double*>(ring_smem + (((size_t)A.PB * NC2 * sizeof(T) + 15) & ~(size_t)15));
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
     if ((int)blockIdx.x >= nE) return;
     if (threadIdx.x == 0) {
         dead = 0;
-        for (int q = 0; q < kRing; q++) {
+        for (int q = 0; q < kRingSlots; q++) {
             bar_init(full + q);
             bar_init(empty + q);
         }
@@ -255,10 +258,10 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
             const int total = __shfl_sync(~0u, sum, 31);
             int done = 0, freed = 0;  // of these 32: requested; blocks released meanwhile
             while (done < n) {
-                const bool ok = have && lane >= done && used + sum - freed <= A.PB && k - tail < kRing;
+                const bool ok = have && lane >= done && used + sum - freed <= A.PB && ring_may_request(k, tail, A.NG);
                 const unsigned m = __ballot_sync(~0u, ok);
                 if (ok) {
-                    const int q = k % kRing;
+                    const int q = k % kRingSlots;
                     int blk = (next + sum - cnt) % A.PB;
                     first[q] = blk;
                     cnts[q] = cnt;
@@ -279,14 +282,14 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
                 if (m == 0u) {  // no room: wait for the oldest position in flight
                     bool got = false;
                     for (int it = 0; it < kBarPolls && !got; it++) {
-                        got = __all_sync(~0u, bar_test(empty + tail % kRing, (unsigned)(tail / kRing) & 1u));
+                        got = __all_sync(~0u, bar_test(empty + tail % kRingSlots, ring_lap_parity(tail)));
                         if (__any_sync(~0u, dead != 0)) break;
                     }
                     if (!got) {
                         fail = true;
                         break;
                     }
-                    freed += cnts[tail % kRing];
+                    freed += cnts[tail % kRingSlots];
                     tail++;
                     // the positions' shared reads come before the copies that reuse their blocks
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -306,7 +309,7 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
         }
         // no copy may be in flight when the thread block ends
         for (int k = tail; k < head; k++)
-            for (int it = 0; it < kBarPolls && !bar_test(full + k % kRing, (unsigned)(k / kRing) & 1u); it++) {
+            for (int it = 0; it < kBarPolls && !bar_test(full + k % kRingSlots, ring_lap_parity(k)); it++) {
             }
         return;
     }
@@ -328,7 +331,7 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
     int4 nb_cur = v < nV ? early(A.swNb + v) : make_int4(-1, -1, -1, -1);
     while (v < nV) {
         const bool bwd = v >= nE;
-        const int i = i_cur, q = k % kRing;
+        const int i = i_cur, q = k % kRingSlots;
         const int4 nbv = nb_cur;
         const int vn = position(k + A.NG, nE);
         if (vn < nV) {  // the next program entry, in flight during this position
@@ -355,8 +358,11 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
         // the position's blocks have arrived
         bool got = false;
         for (int it = 0; it < kBarPolls && !got; it++) {
-            got = __all_sync(~0u, bar_test(full + q, (unsigned)(k / kRing) & 1u));
-            if (__any_sync(~0u, dead != 0)) break;
+            got = __all_sync(~0u, bar_test(full + q, ring_lap_parity(k)));
+            if (__any_sync(~0u, dead != 0)) {
+                got = false;
+                break;
+            }
         }
         if (!got) {
             dead = 1;
