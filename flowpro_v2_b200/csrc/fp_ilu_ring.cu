@@ -21,8 +21,9 @@
 //
 // Measured per application, us, before (staged whole positions, the groups' number timed on the
 // first application) and now: 18,000 tetrahedra of 50 unknowns FP64 950 -> 420, 86,700 FP32
-// 2,200 -> 1,010 (4.3 GB: 4.3 TB/s), 8,832 triangles of 30 unknowns FP32 725 -> 434, 12 merged cases
-// of 12 unknowns 1,050 -> 571, 4 of 40 unknowns 1,250 -> 575.
+// 2,200 -> 1,005 (4.3 GB: 4.3 TB/s), 8,832 triangles of 30 unknowns FP32 725 -> 434, 12 merged cases
+// of 12 unknowns 1,050 -> 571, 4 of 40 unknowns 1,250 -> 583; 80 merged cases of 12 unknowns, 1.28
+// million triangles, over 100 pseudo-time steps with the finished ones passing through 1,900 -> 1,100.
 //
 // A producer warp requests the factor blocks of the coming positions as single bulk copies into
 // a ring of blocks in position order, as far ahead as the ring has room (10 blocks of 50 x 50 in
@@ -75,6 +76,13 @@ struct Cfg {
     static_assert(NC % 2 == 0 && RL * CPW <= 32 && NC <= 32 * WG && P % WG == 0, "lanes of the row split");
     // two thread blocks per SM for the small blocks, whose positions are short
     static constexpr int CTAS = NC <= 32 ? 2 : 1;
+    static constexpr size_t WORK = ((size_t)GROUPS * PART + (size_t)WARPS * WV) * sizeof(double);  // sums and values
+    // blocks of the ring: what is left of 226 KB (one thread block per SM) or 112 KB (two) beside
+    // the work arrays and the static shared memory; a position takes up to 1 + nf blocks
+    static constexpr int PB = (int)std::min<size_t>(kMaxBlocks, ((CTAS == 1 ? 224 : 110) * 1024 - WORK) / ((size_t)NC * NC * sizeof(T)));
+    static_assert(PB >= 1 + kFaces, "the ring holds a position");
+    static constexpr size_t RING = ((size_t)PB * NC * NC * sizeof(T) + 15) & ~(size_t)15;
+    static constexpr size_t SMEM = RING + WORK;
     // the G sums of a row (p: [P][NC] partial sums, h halves added), in the order of the chains above
     __device__ static __forceinline__ double row(const double* p, int r) {
         if constexpr (G == 2) return (p[r] + p[NC + r]) + (p[2 * NC + r] + p[3 * NC + r]);
@@ -98,6 +106,16 @@ __device__ __forceinline__ bool bar_test(unsigned long long* b, unsigned parity)
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
+        : "=r"(ok)
+        : "r"(sa(b)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// the same without suspending the thread
+__device__ __forceinline__ bool bar_passed(unsigned long long* b, unsigned parity) {
+    unsigned ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n}"
         : "=r"(ok)
         : "r"(sa(b)), "r"(parity)
         : "memory");
@@ -129,7 +147,7 @@ __device__ __forceinline__ int position(int k, int nE) {
 }
 
 struct SweepArgs {
-    int nf, ld, nE, PB, NG;   // PB: blocks of the ring, NG: elements in flight per thread block
+    int nf, ld, nE, NG;       // NG: elements in flight per thread block
     const int* swEl;          // [2 nE] element at a position
     const int4* swNb;         // [2 nE] neighbours multiplied there (-1 none)
     const double* b;          // [NC][ld]
@@ -212,14 +230,14 @@ __device__ __forceinline__ void group_sync(int grp) {
 template <class T, int NC>
 __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS) k_sweep_ring(SweepArgs A, const T* __restrict__ F) {
     using C = Cfg<T, NC>;
-    constexpr int NC2 = NC * NC;
+    constexpr int NC2 = NC * NC, PB = C::PB;
     extern __shared__ __align__(128) unsigned char ring_smem[];
     __shared__ __align__(8) unsigned long long full[kRingSlots], empty[kRingSlots];
     __shared__ int first[kRingSlots];
     __shared__ int cnts[kRingSlots];  // producer's own: blocks of each position
     __shared__ volatile int dead;
     T* ring = reinterpret_cast<T*>(ring_smem);
-    double* work = reinterpret_cast<double*>(ring_smem + (((size_t)A.PB * NC2 * sizeof(T) + 15) & ~(size_t)15));
+    double* work = reinterpret_cast<double*>(ring_smem + C::RING);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nE = A.nE, nf = A.nf, nV = 2 * nE;
     if ((int)blockIdx.x >= nE) return;
@@ -234,21 +252,34 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
     __syncthreads();
 
     if (warp == C::WARPS) {  // ------------------------------------------------ producer
+        // A trip takes all positions that have been released since the last one: lane l tests the barrier of
+        // position tail + l, their blocks are added up, one proxy fence, and as many of the next 32
+        // positions as now fit are requested, a lane each.  With one position a trip the producer
+        // bounded large meshes of small blocks at 1,150 cycles a position (an application, all cases live,
+        // ms: 1.28 million triangles of 12 unknowns 5.09 -> 2.05, 1.34 million of 24 5.35 -> 3.33; the 100
+        // pseudo-time steps of the former 43.6 -> 20.3 s).
         const int ns = 1 + nf;
         int head = 0, tail = 0;        // positions requested, released
         int used = 0, next = 0;        // blocks in use, first free block
         bool more = true, fail = false;
+        int i_next = 0;
+        int4 nb_next = make_int4(-1, -1, -1, -1);
+        auto fetch = [&](int k) {  // the program entry of position k, used a trip later
+            const int v = position(k, nE);
+            if (v >= nV) return;
+            i_next = early(A.swEl + v);
+            nb_next = early(A.swNb + v);
+        };
+        fetch(lane);
         while (more && !fail) {
             const int k = head + lane, v = position(k, nE);
             const bool have = v < nV;
-            int i = 0, cnt = 0;
-            int4 nb = make_int4(-1, -1, -1, -1);
-            if (have) {
-                i = A.swEl[v];
-                nb = A.swNb[v];
-                if (!(A.live && !A.live[A.caseOf[i]]))
-                    cnt = (v >= nE) + (nb.x >= 0) + (nb.y >= 0) + (nb.z >= 0) + (nb.w >= 0);
-            }
+            const int i = i_next;
+            const int4 nb = nb_next;
+            fetch(k + 32);
+            int cnt = 0;
+            if (have && !(A.live && !A.live[A.caseOf[i]]))
+                cnt = (v >= nE) + (nb.x >= 0) + (nb.y >= 0) + (nb.z >= 0) + (nb.w >= 0);
             int sum = cnt;  // blocks up to and with this position
             for (int o = 1; o < 32; o <<= 1) {
                 const int t = __shfl_up_sync(~0u, sum, o);
@@ -257,12 +288,12 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
             const int n = __popc(__ballot_sync(~0u, have));
             const int total = __shfl_sync(~0u, sum, 31);
             int done = 0, freed = 0;  // of these 32: requested; blocks released meanwhile
-            while (done < n) {
-                const bool ok = have && lane >= done && used + sum - freed <= A.PB && ring_may_request(k, tail, A.NG);
+            while (true) {
+                const bool ok = have && lane >= done && used + sum - freed <= PB && ring_may_request(k, tail, A.NG);
                 const unsigned m = __ballot_sync(~0u, ok);
                 if (ok) {
                     const int q = k % kRingSlots;
-                    int blk = (next + sum - cnt) % A.PB;
+                    int blk = (next + sum - cnt) % PB;
                     first[q] = blk;
                     cnts[q] = cnt;
                     bar_expect(full + q, (unsigned)(cnt * NC2 * sizeof(T)));
@@ -273,30 +304,37 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
                         for (int f = -1; f < kFaces; f++)
                             if (f < 0 ? v >= nE : nbs[f < 0 ? 0 : f] >= 0) {
                                 copy_block(ring + (size_t)blk * NC2, src + (size_t)(1 + f) * NC2, NC2 * sizeof(T), full + q);
-                                blk = blk + 1 == A.PB ? 0 : blk + 1;
+                                blk = blk + 1 == PB ? 0 : blk + 1;
                             }
                     }
                 }
                 __syncwarp();
                 done += __popc(m);
-                if (m == 0u) {  // no room: wait for the oldest position in flight
-                    bool got = false;
-                    for (int it = 0; it < kBarPolls && !got; it++) {
-                        got = __all_sync(~0u, bar_test(empty + tail % kRingSlots, ring_lap_parity(tail)));
-                        if (__any_sync(~0u, dead != 0)) break;
-                    }
-                    if (!got) {
-                        fail = true;
-                        break;
-                    }
-                    freed += cnts[tail % kRingSlots];
-                    tail++;
-                    // the positions' shared reads come before the copies that reuse their blocks
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                if (done == n) break;
+                // no room for the next one: wait for the oldest position in flight, then take all those that
+                // follow it and are released (polling the 32 barriers for the first of them cost the
+                // other warps 5 % where the chain of levels bounds: shared memory is theirs)
+                bool got = false;
+                for (int it = 0; it < kBarPolls && !got; it++) {
+                    got = __all_sync(~0u, bar_test(empty + tail % kRingSlots, ring_lap_parity(tail)));
+                    if (__any_sync(~0u, dead != 0)) break;
                 }
+                if (!got) {
+                    fail = true;
+                    break;
+                }
+                const int t = tail + lane;
+                const bool rel = t < head + done && bar_passed(empty + t % kRingSlots, ring_lap_parity(t));
+                int run = __ffs(~__ballot_sync(~0u, rel)) - 1;  // -1: all 32
+                if (run < 0) run = 32;
+                freed += __reduce_add_sync(~0u, lane < run ? cnts[(tail + lane) % kRingSlots] : 0);
+                tail += run;
+                // the positions' shared reads come before the copies that reuse their blocks
+                __syncwarp();
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             }
             used += total - freed;
-            next = (next + total) % A.PB;
+            next = (next + total) % PB;
             head += done;
             more = n == 32;
         }
@@ -397,7 +435,7 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
         __syncwarp();
         int blk = first[q];
         const T* D = ring + (size_t)blk * NC2;
-        if (bwd) blk = blk + 1 == A.PB ? 0 : blk + 1;
+        if (bwd) blk = blk + 1 == PB ? 0 : blk + 1;
         if (!skip) {
             // the position's blocks follow one another in the ring, in the order of the faces
             double sf[kFaces][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
@@ -407,7 +445,7 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
                 if (nbs[f] >= 0) {
                     if (act && got && (C::H == 1 || f / 2 == h))
                         rows_times<T, NC, 2>(ring + (size_t)blk * NC2, wv + (f - f0) * C::WC + (g - g0) * C::CW, 2 * rl, g, sf[f]);
-                    blk = blk + 1 == A.PB ? 0 : blk + 1;
+                    blk = blk + 1 == PB ? 0 : blk + 1;
                 }
             double* p = part + buf * C::P * NC;
             buf ^= 1;
@@ -463,18 +501,8 @@ __global__ void __launch_bounds__(32 * (Cfg<T, NC>::WARPS + 1), Cfg<T, NC>::CTAS
 template <class T, int NC>
 struct Ring {
     using C = Cfg<T, NC>;
-    static constexpr size_t kWork = ((size_t)Cfg<T, NC>::GROUPS * Cfg<T, NC>::PART + (size_t)C::WARPS * Cfg<T, NC>::WV) * sizeof(double);
-    static size_t smem(int PB) { return (((size_t)PB * NC * NC * sizeof(T) + 15) & ~(size_t)15) + kWork; }
-    // blocks of the ring: what is left of 226 KB (one thread block per SM) or 112 KB (two) beside
-    // the work arrays and the static shared memory; a position takes up to 1 + nf blocks
-    static int blocks() {
-        const size_t room = (size_t)(Cfg<T, NC>::CTAS == 1 ? 224 : 110) * 1024 - kWork;
-        return (int)std::min<size_t>(kMaxBlocks, room / ((size_t)NC * NC * sizeof(T)));
-    }
     static int configure(fp_ctx* c, int pi) {
-        const int PB = blocks();
-        if (PB < 1 + kFaces) return set_err(c, FP_ERR_UNSUPPORTED, "block ILU(0): the sweep's ring does not fit an SM");
-        const size_t sm = smem(PB);
+        constexpr size_t sm = C::SMEM;
         int rc, dev = 0, nsm = 0, perSm = 0;
         if ((rc = cuda_check(c, cudaFuncSetAttribute(k_sweep_ring<T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
                              "smem")))
@@ -486,23 +514,23 @@ struct Ring {
             return rc;
         if (perSm < 1) return set_err(c, FP_ERR_UNSUPPORTED, "block ILU(0): the sweep does not fit an SM");
         c->ring_grid[pi] = std::max(1, std::min(c->hm.nElem, nsm * perSm));
-        c->ring_blocks[pi] = PB;
         return FP_OK;
     }
     static cudaError_t launch(fp_ctx* c, int pi, SweepArgs& a, const T* F) {
-        a.PB = c->ring_blocks[pi];
         if (a.NG <= 0) {
             // elements in flight for six levels of average width: with more, the warps that wait
             // several levels ahead poll the L2 for nothing (8,832 triangles of 30 unknowns, 62 a
             // level: 434 us with 1 or 2 a thread block, 508 with 8; 53,400 of 12 unknowns, 196 a
-            // level: 775, 571 and 594 us with 1, 4 and 16)
+            // level: 775, 571 and 594 us with 1, 4 and 16).  Large meshes keep every warp busy: 1.28
+            // million of 12 unknowns 4.23, 2.45 and 2.05 ms with 4, 8 and 16, 1.34 million of 24 4.54 and
+            // 3.33 with 4 and 8.
             const double width = (double)a.nE / std::max<size_t>(1, c->lvlF_ptr.size() - 1);
             a.NG = 1 + (int)std::min(64.0, 6.0 * width / c->ring_grid[pi]);
         }
         a.NG = std::min(a.NG, C::GROUPS);
         void* args[] = {&a, (void*)&F};
         return cudaLaunchCooperativeKernel((const void*)k_sweep_ring<T, NC>, dim3(c->ring_grid[pi]), dim3(32 * (C::WARPS + 1)), args,
-                                           smem(a.PB), c->stream);
+                                           C::SMEM, c->stream);
     }
 };
 
