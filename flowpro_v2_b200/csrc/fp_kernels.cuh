@@ -145,6 +145,8 @@ struct Element {
         const double* tab = M.tab;
         const double* phiL = tab + TB::o_phiL + (k * NQF + p) * NB;
         const double* dphiL = tab + TB::o_dphiL + (k * NQF + p) * NB * DIM;
+        double u[DIM], X[DIM];
+        point_motion(M, e, k, p, u, X);
         // traces (DGpure.java:239-264)
         constexpr int NG = GRAD ? DIM * NE : 1;
         T WL[NE], WR[NE], dWL[NG], dWR[NG];
@@ -153,8 +155,10 @@ struct Element {
             const double* phiR = tab + TB::o_phiR + ((kr_face * NP + pm) * NQF + p) * NB;
             const double* dphiR = tab + TB::o_dphiR + ((kr_face * NP + pm) * NQF + p) * NB * DIM;
             trace<GRAD>(phiR, dphiR, JinvR, [&](int c) { return nbl(c, TT); }, WR, dWR);
+        } else {
+            boundary_trace<GRAD>(M, e, TT, n, u, X, WL, WR, dWL, dWR);
         }
-        point_flux<GRAD>(M, e, k, p, TT, n, dL, eps_e, eps_nb, WL, WR, dWL, dWR, C, Jmp);
+        trace_flux<GRAD>(M, TT, n, dL, eps_e, eps_nb, u, WL, WR, dWL, dWR, C, Jmp);
     }
 
     // value and (GRAD) physical gradient of the coefficients coef(c) at one point
@@ -203,47 +207,63 @@ struct Element {
         }
     }
 
-    // the integrand of face_point from the traces WL and, on interior faces, WR (dWL, dWR with GRAD)
-    template <bool GRAD, class T>
-    static __device__ __forceinline__ void point_flux(const DevMesh& M, int e, int k, int p, int TT, const double* n, double dL,
-                                                      double eps_e, double eps_nb, T* WL, T* WR, T* dWL, T* dWR, T* C, T* Jmp) {
+    // mesh velocity u and position X at the face point (Element.java:299-332)
+    static __device__ __forceinline__ void point_motion(const DevMesh& M, int e, int k, int p, double* u, double* X) {
         const int ld = M.ld;
-        const double* geo = M.geo;
-        const double* tab = M.tab;
-        const fp_model_params& P = M.P;
-        const bool interior = TT > -1;
-        // mesh velocity and position at the face point (Element.java:299-332)
-        double u[DIM];
 #pragma unroll
         for (int d = 0; d < DIM; d++) u[d] = 0;
         if (M.vu != nullptr) {
 #pragma unroll
             for (int i = 0; i < NVF; i++) {
-                const double li = ldg(tab + TB::o_finterp + p * NVF + i);
+                const double li = ldg(M.tab + TB::o_finterp + p * NVF + i);
                 const int v = face_vertex<DIM>(k, i);
 #pragma unroll
                 for (int d = 0; d < DIM; d++) u[d] += li * ldg(M.vu + (size_t)(v * DIM + d) * ld + e);
             }
         }
-        double X[DIM];
         if (Mdl::NE == 1) {  // only the scalar test equation's boundary values use the position
-            const double* xi = tab + TB::o_xiL + (k * NQF + p) * DIM;
+            const double* xi = M.tab + TB::o_xiL + (k * NQF + p) * DIM;
 #pragma unroll
             for (int i = 0; i < DIM; i++) {
                 double s = 0;
 #pragma unroll
-                for (int j = 0; j < DIM; j++) s += ldg(geo + (size_t)(GL::JM + i * DIM + j) * ld + e) * ldg(xi + j);
-                X[i] = s + ldg(geo + (size_t)(GL::X0 + i) * ld + e);
+                for (int j = 0; j < DIM; j++) s += ldg(M.geo + (size_t)(GL::JM + i * DIM + j) * ld + e) * ldg(xi + j);
+                X[i] = s + ldg(M.geo + (size_t)(GL::X0 + i) * ld + e);
             }
         }
-        if (!interior) {
-            // the outlet pressure of the element's case in a batch of cases, else the model's
-            Mdl::boundaryValue(WL, n, TT, u, X, WR, P, M.case_pout ? ldg(M.case_pout + M.case_of[e]) : P.p_out);
-            if constexpr (GRAD) {
+    }
+
+    // the other side's trace on a boundary face
+    template <bool GRAD, class T>
+    static __device__ __forceinline__ void boundary_trace(const DevMesh& M, int e, int TT, const double* n, const double* u,
+                                                          const double* X, T* WL, T* WR, const T* dWL, T* dWR) {
+        // the outlet pressure of the element's case in a batch of cases, else the model's
+        Mdl::boundaryValue(WL, n, TT, u, X, WR, M.P, M.case_pout ? ldg(M.case_pout + M.case_of[e]) : M.P.p_out);
+        if constexpr (GRAD) {
 #pragma unroll
-                for (int i = 0; i < DIM * NE; i++) dWR[i] = dWL[i];
-            }
+            for (int i = 0; i < DIM * NE; i++) dWR[i] = dWL[i];
         }
+    }
+
+    // the integrand of face_point from the traces WL and, on interior faces, WR (dWL, dWR with GRAD)
+    template <bool GRAD, class T>
+    static __device__ __forceinline__ void point_flux(const DevMesh& M, int e, int k, int p, int TT, const double* n, double dL,
+                                                      double eps_e, double eps_nb, T* WL, T* WR, T* dWL, T* dWR, T* C, T* Jmp) {
+        double u[DIM], X[DIM];
+        point_motion(M, e, k, p, u, X);
+        if (TT < 0) boundary_trace<GRAD>(M, e, TT, n, u, X, WL, WR, dWL, dWR);
+        trace_flux<GRAD>(M, TT, n, dL, eps_e, eps_nb, u, WL, WR, dWL, dWR, C, Jmp);
+    }
+
+    // the same from both sides' traces.  face_point branches once over the kind of face: with the
+    // neighbour's trace and the boundary's in two conditions ptxas spills a third more in the viscous face
+    // pass (84 -> 116 bytes at 24 unknowns, 99 -> 105 us on 200,568 triangles).
+    template <bool GRAD, class T>
+    static __device__ __forceinline__ void trace_flux(const DevMesh& M, int TT, const double* n, double dL, double eps_e,
+                                                      double eps_nb, const double* u, T* WL, T* WR, const T* dWL, const T* dWR,
+                                                      T* C, T* Jmp) {
+        const fp_model_params& P = M.P;
+        const bool interior = TT > -1;
         // inviscid flux (DGpure.java:266-281)
         double vn = 0;
 #pragma unroll
