@@ -1,11 +1,17 @@
 // Large copies between device memory and pageable host memory.
 //
 // A pageable copy goes through the driver's staging buffer on one thread, which also takes the page
-// faults of a fresh destination: 38 MB (200,568 triangles of 24 unknowns) took 8.2 ms down, where the
-// link needs 0.8.  Here the chunks go through pinned staging slots while several threads copy
-// between the slots and the caller's memory, each its slice of every chunk: 2.6 ms.  Copies below
+// faults of a fresh destination: 38 MB (200,568 triangles of 24 unknowns) took 8.2 to 17 ms down,
+// where the link needs 0.8.  Here the chunks go through pinned staging slots while several threads copy
+// between the slots and the caller's memory, each its slice of every chunk: 2.45 ms.  Copies below
 // kLeastBytes, pinned host memory and calls that find the staging memory in use by another thread take
 // the plain cudaMemcpyAsync.
+//
+// The slots are small because pinning them is part of the first large copy of a program that has one
+// context at a time: 12 MB take 5.0 to 8.4 ms to allocate and 1.4 to free, 6 MB 2.7 to 5.7 and 0.9.
+// State of 38 MB down / up, ms: 6 slots of 2 MB 2.5 / 2.3, 6 of 1 MB 2.45 / 2.1, 4 of 1 MB 2.65 / 1.85, 3 of
+// 1 MB 3.0 / 1.7, 6 of 512 KB 2.8 / 1.8.  The threads exist only while the link is at work: the stream's
+// earlier work is waited for first.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -20,7 +26,7 @@ namespace fp {
 
 namespace {
 
-constexpr size_t kSlotBytes = (size_t)2 << 20;
+constexpr size_t kSlotBytes = (size_t)1 << 20;
 constexpr int kSlots = 6;
 constexpr size_t kLeastBytes = (size_t)2 << 20;
 constexpr unsigned kMostThreads = 8;
@@ -100,7 +106,7 @@ struct Copiers {
 };
 
 // the copy through the staging slots; *taken false: not applicable here, nothing has been copied
-int staged(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* taken) {
+int staged_copy(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* taken) {
     *taken = false;
     if (bytes < kLeastBytes || !pageable(host)) return FP_OK;
     Staging& S = staging();
@@ -111,44 +117,43 @@ int staged(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* take
         S.buf = nullptr;
         return FP_OK;
     }
+    // before any thread waits for a chunk: on the caller's stream the work ahead may be long
+    int rc = cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
+    if (rc) return rc;
+    Copiers C((char*)host, S.buf, bytes, down);
     cudaEvent_t ev[kSlots] = {};
-    int rc = FP_OK;
     for (auto& e : ev)
         if (!rc) rc = cuda_check(c, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
-    if (!rc) {
-        Copiers C((char*)host, S.buf, bytes, down);
-        const unsigned hw = std::thread::hardware_concurrency();
-        if (!C.start((int)std::max(1u, std::min(kMostThreads, hw / 2)))) {
-            for (auto& e : ev) cudaEventDestroy(e);
-            return FP_OK;
-        }
+    auto slot = [&](int k) { return S.buf + (size_t)(k % kSlots) * kSlotBytes; };
+    auto at = [&](int k) { return (char*)dev + (size_t)k * kSlotBytes; };
+    auto transfer = [&](int k) {  // chunk k between its slot and the device
+        void *to = down ? slot(k) : at(k), *from = down ? at(k) : slot(k);
+        rc = cuda_check(c, cudaMemcpyAsync(to, from, C.size(k), down ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, c->stream),
+                        down ? "download" : "upload");
+        if (!rc) rc = cuda_check(c, cudaEventRecord(ev[k % kSlots], c->stream), "event");
+    };
+    int issued = 0;
+    if (down)  // on their way while the threads start
+        for (; issued < std::min(C.chunks, kSlots) && !rc; issued++) transfer(issued);
+    const unsigned hw = std::thread::hardware_concurrency();
+    if (!rc && C.start((int)std::max(1u, std::min(kMostThreads, hw / 2)))) {
         *taken = true;
-        auto slot = [&](int k) { return S.buf + (size_t)(k % kSlots) * kSlotBytes; };
-        auto at = [&](int k) { return (char*)dev + (size_t)k * kSlotBytes; };
         if (down) {
-            int issued = 0;
             for (int k = 0; k < C.chunks && !rc; k++) {
                 while (issued < C.chunks && issued < k + kSlots && !rc) {
-                    if (issued >= kSlots) {
-                        if (issued > k && !C.finished(issued - kSlots)) break;  // later: chunk k is on its way
-                        C.await(issued - kSlots);
-                    }
-                    rc = cuda_check(c, cudaMemcpyAsync(slot(issued), at(issued), C.size(issued), cudaMemcpyDeviceToHost, c->stream),
-                                    "download");
-                    if (!rc) rc = cuda_check(c, cudaEventRecord(ev[issued % kSlots], c->stream), "event");
-                    issued++;
+                    if (issued > k && !C.finished(issued - kSlots)) break;  // later: chunk k is on its way
+                    C.await(issued - kSlots);
+                    transfer(issued++);
                 }
                 if (!rc) rc = cuda_check(c, cudaEventSynchronize(ev[k % kSlots]), "sync");
                 if (!rc) C.open.store(k + 1, std::memory_order_release);
             }
-            if (!rc) C.await(C.chunks - 1);
-            for (int k = 0; k < C.chunks && !rc; k++) C.await(k);
+            for (int k = std::max(0, C.chunks - kSlots); k < C.chunks && !rc; k++) C.await(k);
         } else {
             C.open.store(std::min(C.chunks, kSlots), std::memory_order_release);
             for (int k = 0; k < C.chunks && !rc; k++) {
                 C.await(k);
-                rc = cuda_check(c, cudaMemcpyAsync(at(k), slot(k), C.size(k), cudaMemcpyHostToDevice, c->stream), "upload");
-                if (!rc) rc = cuda_check(c, cudaEventRecord(ev[k % kSlots], c->stream), "event");
+                transfer(k);
                 if (!rc && k >= 1) {  // the slot of chunk k - 1 takes chunk k - 1 + kSlots
                     rc = cuda_check(c, cudaEventSynchronize(ev[(k - 1) % kSlots]), "sync");
                     C.open.store(std::min(C.chunks, k + kSlots), std::memory_order_release);
@@ -157,11 +162,22 @@ int staged(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* take
             // the slots are free again when the last copies have left them
             if (!rc) rc = cuda_check(c, cudaEventSynchronize(ev[(C.chunks - 1) % kSlots]), "sync");
         }
-        if (rc) cudaStreamSynchronize(c->stream);  // no copy may use the slots after this
     }
+    if (rc || !*taken) cudaStreamSynchronize(c->stream);  // no copy may use the slots after this
     for (auto& e : ev)
         if (e) cudaEventDestroy(e);
     return rc;
+}
+
+// the same without exceptions: what can throw (host memory for the bookkeeping, the lock) does so before the
+// first transfer
+int staged(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* taken) {
+    try {
+        return staged_copy(c, host, dev, bytes, down, taken);
+    } catch (...) {
+        *taken = false;
+        return FP_OK;
+    }
 }
 
 }  // namespace
