@@ -110,9 +110,7 @@ void free_all(fp_ctx* c) {
     for (double* p : c->allocs) cudaFree(p);
     c->allocs.clear();
     if (c->h_scal) cudaFreeHost(c->h_scal);
-    c->h_scal = nullptr;
-    if (c->h_part) cudaFreeHost(c->h_part);
-    c->h_part = nullptr;
+    c->h_scal = c->h_part = nullptr;
     c->d_Adiag = c->d_Aneigh = c->d_rhs = c->d_KT = c->d_P64 = nullptr;
     c->d_mass = nullptr;
     c->d_vu = nullptr;
@@ -154,6 +152,18 @@ __global__ void k_from_soa(int nElem, int ld, int nc, const double* __restrict__
     if (t >= (size_t)nElem * nc) return;
     const int e = (int)(t / nc), cc = (int)(t - (size_t)e * nc);
     out[t] = in[(size_t)cc * ld + e];
+}
+
+// every coefficient of equation m at v[m], in all three time levels
+struct ConstState {
+    double v[8];
+};
+__global__ void k_const_state(int nElem, int ld, int nb, ConstState w0, double* __restrict__ W, double* __restrict__ Wo,
+                              double* __restrict__ Wo2) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nElem) return;
+    const size_t i = (size_t)blockIdx.y * ld + e;
+    W[i] = Wo[i] = Wo2[i] = w0.v[blockIdx.y / nb];
 }
 
 int host_to_soa(fp_ctx* c, const double* h, double* d) {
@@ -460,9 +470,10 @@ int fp_mesh_upload(fp_ctx* c, const fp_mesh_desc* desc, const fp_model_params* m
     size_t npart = std::max<size_t>(npelem, (size_t)592 * 201);
     if ((rc = dalloc(c, &c->d_part, npart)) || (rc = dalloc(c, &c->d_scal, 1024)) || (rc = dalloc(c, &c->d_status, 4)))
         return rc;
-    if (cudaMallocHost(&c->h_scal, 1024 * sizeof(double)) != cudaSuccess ||
-        cudaMallocHost(&c->h_part, npelem * sizeof(double)) != cudaSuccess)
+    // one pinned allocation: each takes 1 to 3 ms, whatever its size
+    if (cudaMallocHost(&c->h_scal, (1024 + npelem) * sizeof(double)) != cudaSuccess)
         return set_err(c, FP_ERR_CUDA, "cudaMallocHost");
+    c->h_part = c->h_scal + 1024;
     rc = cuda_check(c, cudaStreamSynchronize(c->stream), "upload sync");
     if (rc) return rc;
     c->has_mesh = true;
@@ -542,15 +553,11 @@ int fp_state_get(fp_ctx* c, int which, double* w) {
 int fp_state_init_const(fp_ctx* c) {
     int rc = need_mesh(c);
     if (rc) return rc;
-    double w0[8];
-    const_init_condition(c->hm.model, w0);
-    const int nb = c->hm.tab.nb, ne = c->hm.model.n_eqs;
-    std::vector<double> h((size_t)c->hm.nElem * c->nc);
-    for (int e = 0; e < c->hm.nElem; e++)
-        for (int m = 0; m < ne; m++)
-            for (int j = 0; j < nb; j++) h[(size_t)e * c->nc + m * nb + j] = w0[m];
-    for (int which = 0; which < 3; which++)
-        if ((rc = host_to_soa(c, h.data(), state_ptr(c, which)))) return rc;
+    ConstState w0;
+    const_init_condition(c->hm.model, w0.v);
+    const dim3 grid((unsigned)((c->hm.nElem + 255) / 256), (unsigned)c->nc);
+    k_const_state<<<grid, 256, 0, c->stream>>>(c->hm.nElem, c->hm.ld, c->hm.tab.nb, w0, c->d_W, c->d_Wo, c->d_Wo2);
+    if ((rc = cuda_check(c, cudaGetLastError(), "constant state"))) return rc;
     return cuda_check(c, cudaStreamSynchronize(c->stream), "sync");
 }
 
