@@ -27,13 +27,15 @@ namespace {
 
 constexpr int kRT = 256;
 
-// Elements per chunk of the segmented reductions, a power of two: small enough that the chunks of a
-// few small cases still fill the GPU (16,600 triangles of 40 unknowns: 2,048 elements a chunk were 10
-// thread blocks and 267 us a dot product pass, 64 are 260 and 16 us), large enough that the partial
-// sums of many cases stay few.
-inline int chunk_elements(int nElem) {
+// Elements per chunk of a case's segmented reductions, a power of two from the size of the case alone, so
+// that its sums, and its solution, do not depend on the cases it is merged with.  Up to 128 chunks a
+// case: small ones still fill the GPU (four of 40 unknowns, 16,600 triangles, a solve's Krylov work: 3.9 ms
+// with up to 128, 4.9 with 64, 7.0 with 32; chunks of 2,048 elements were 35.6), and large groups have
+// work in every thread block (91 cases, 1.6 million triangles of 40 unknowns: 1.99 ms an iteration, 2.24
+// with chunks of 2,048).
+inline int chunk_elements(int caseElem) {
     int n = 64;
-    while (n < 2048 && nElem / n > 8 * 148) n *= 2;
+    while (n < 2048 && caseElem / n > 128) n *= 2;
     return n;
 }
 
@@ -236,10 +238,10 @@ struct Batch {
 int batch_prepare(fp_ctx* c, int kmax) {
     const int n = c->n_cases;
     if (c->batch_ready && c->batch_kmax >= kmax) return FP_OK;
-    const int chunk = chunk_elements(c->hm.nElem);
     std::vector<int> e0, e1, cptr(n + 1, 0);
     for (int cs = 0; cs < n; cs++) {
         cptr[cs] = (int)e0.size();
+        const int chunk = chunk_elements(c->case_e0[cs + 1] - c->case_e0[cs]);
         for (int a = c->case_e0[cs]; a < c->case_e0[cs + 1]; a += chunk) {
             e0.push_back(a);
             e1.push_back(std::min(a + chunk, c->case_e0[cs + 1]));
