@@ -104,12 +104,12 @@ struct fp_ctx {
     unsigned ilu_epoch = 0;          // epoch of the last application
     unsigned ilu_fepoch = 0;         // epoch of the last factorisation
     int ilu_max_polls = 1 << 19;     // poll limit of every dependency wait of the ILU kernels
+    enum PubWords { PUB_UNKNOWN, PUB_REGISTER, PUB_RING } pub_words = PUB_UNKNOWN;  // whose words d_ilu_pub holds
     unsigned long long* d_ilu_pub = nullptr;  // [4 nElem nc] published sweep values (forward, backward; two words each, or two halves)
     int sweep_grid = 0;           // thread blocks of the persistent sweep kernel
-    // streamed sweep kernel: grid per factor precision [FP64, FP32] (0: not configured yet), whether
-    // d_ilu_pub holds its words, and which half is next
+    // streamed sweep kernel: grid per factor precision [FP64, FP32] (0: not configured yet), and which half
+    // of d_ilu_pub is next
     int ring_grid[2] = {0, 0};
-    bool ring_pub_ready = false;
     int ring_parity = 0;
     int sweep_variant = 0;           // 0 streamed, 1 register, 2-6 streamed with 1-16 elements in flight per block
     // Krylov

@@ -404,7 +404,7 @@ int ilu_build(fp_ctx* c) {
     c->sweep_grid = std::max(1, std::min(nE, nsm * std::max(1, std::min(perSm, perSm32))));
     c->ilu_epoch = 0;
     c->ilu_fepoch = 0;
-    c->ring_pub_ready = false;
+    c->pub_words = fp_ctx::PUB_REGISTER;  // cleared above
     c->ring_parity = 0;
     c->ilu_built = true;
     return FP_OK;
@@ -502,7 +502,7 @@ void ilu_release(fp_ctx* c) {
     c->d_ilu_pub = nullptr;
     c->sweep_grid = 0;
     c->ring_grid[0] = c->ring_grid[1] = 0;
-    c->ring_pub_ready = false;
+    c->pub_words = fp_ctx::PUB_UNKNOWN;
     c->ring_parity = 0;
 
     c->lvlF_ptr.clear();
@@ -550,11 +550,11 @@ static int launch_register(fp_ctx* c, const T* F, const double* b, double* xx) {
     int nc = c->nc, nf = c->hm.nf, ld = c->hm.ld, nE = c->hm.nElem;
     const size_t words = 2 * (size_t)nE * nc;
     unsigned epoch = ++c->ilu_epoch;
-    if (epoch == 0 || c->ring_pub_ready) {  // wrapped, or words of the other kernel: clear them and start again
+    if (epoch == 0 || c->pub_words != fp_ctx::PUB_REGISTER) {  // wrapped, or not its own words: clear them and start again
         int rc = cuda_check(c, cudaMemsetAsync(c->d_ilu_pub, 0, 2 * words * sizeof(unsigned long long), c->stream), "memset");
         if (rc) return rc;
         epoch = c->ilu_epoch = 1;
-        c->ring_pub_ready = false;
+        c->pub_words = fp_ctx::PUB_REGISTER;
     }
     unsigned long long* pubF = c->d_ilu_pub;
     unsigned long long* pubB = c->d_ilu_pub + words;
@@ -603,7 +603,7 @@ int ilu_check(fp_ctx* c) {
         return rc;
     if (h[0] || h[1]) {
         cudaMemsetAsync(words, 0, sizeof(h), c->stream);
-        c->ring_pub_ready = false;  // what was published is unknown
+        c->pub_words = fp_ctx::PUB_UNKNOWN;
         return set_err(c, FP_ERR_TIMEOUT, "block ILU(0) sweep: a dependency wait gave up");
     }
     return FP_OK;

@@ -561,10 +561,10 @@ bool ring_sweep_applies(int nc) {
 int ring_sweep(fp_ctx* c, int precision, const double* b, double* x, int groups) {
     const size_t n = (size_t)c->hm.nElem * c->nc;
     unsigned long long* pub = c->d_ilu_pub;  // [2][forward, backward][nElem][nc]
-    if (!c->ring_pub_ready) {
+    if (c->pub_words != fp_ctx::PUB_RING) {
         int rc = cuda_check(c, cudaMemsetAsync(pub, 0xff, 4 * n * sizeof(unsigned long long), c->stream), "memset");
         if (rc) return rc;
-        c->ring_pub_ready = true;
+        c->pub_words = fp_ctx::PUB_RING;
     }
     const int par = c->ring_parity;
     c->ring_parity ^= 1;
@@ -586,7 +586,9 @@ int ring_sweep(fp_ctx* c, int precision, const double* b, double* x, int groups)
     a.maxPolls = c->ilu_max_polls;
     a.caseOf = c->batch_mask ? c->d_case_of : nullptr;
     a.live = c->batch_mask ? c->d_blive : nullptr;
-    return precision == FP_PREC_FP32 ? run<float>(c, a, c->d_iluF32) : run<double>(c, a, c->d_iluF64);
+    const int rc = precision == FP_PREC_FP32 ? run<float>(c, a, c->d_iluF32) : run<double>(c, a, c->d_iluF64);
+    if (rc) c->pub_words = fp_ctx::PUB_UNKNOWN;  // not launched: the other half has not been emptied
+    return rc;
 }
 
 }  // namespace fp
