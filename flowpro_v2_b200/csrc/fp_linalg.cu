@@ -454,6 +454,14 @@ int spmv_t(fp_ctx* c, const double* x, double* y) {
     return cuda_check(c, cudaGetLastError(), "spmv_t");
 }
 
+// zeros in the entries [nElem, ld) of every component
+static int clear_padding(fp_ctx* c, double* v) {
+    const size_t ld = c->hm.ld, nE = c->hm.nElem;
+    if (ld == nE) return FP_OK;
+    return cuda_check(
+        c, cudaMemset2DAsync(v + nE, ld * sizeof(double), 0, (ld - nE) * sizeof(double), c->nc, c->stream), "memset");
+}
+
 static int prec_factor_impl(fp_ctx* c, int kind, int precision);
 
 int prec_factor(fp_ctx* c, int kind, int precision) {
@@ -605,6 +613,10 @@ int gmres(fp_ctx* c, int jacobian, int kind, int m, int max_restarts, double tol
     double *w = c->d_w, *aux = c->d_aux, *r = c->d_r, *x = c->d_x, *b = c->d_b;
     double* hs = c->h_scal;
     int total = 0;
+    // The vector kernels run over the padding behind the elements, which the operator and the preconditioner
+    // never write: a solve that met a non-finite value leaves w's there, and every inner product with it.
+    // (The other vectors' padding is written from w, r, b and x, which are clean at the start.)
+    if ((rc = clear_padding(c, w))) return rc;
     // M.apply(r, b); bnrm2 = ||r||
     if ((rc = apply_M(c, kind, b, r)) || (rc = dot(c, r, r, c->d_scal)) || (rc = fetch(c, 1, hs))) return rc;
     double bnrm2 = std::sqrt(hs[0]);
