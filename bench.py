@@ -317,7 +317,7 @@ def ilu_variants(fg, device, box=(100, 34, 34)):
         g = fg.GpuMesh(SOLVE_PROPS, m.vertices, m.elements, tt, m.wall_distance, device=device)
         g.limiter()
         fg.JacobiAssembler(g).assemble_preconditioner(50.0 * g.time_step_bound(), -1, "blockilu0", prec)
-        for v, vname in ((0, "staged_autotuned"), (1, "register"), (2, "staged_1"), (3, "staged_2"), (4, "staged_4")):
+        for v, vname in ((0, "streamed"), (1, "register"), (2, "streamed_1"), (3, "streamed_2"), (4, "streamed_4")):
             try:
                 g.set_ilu_sweep(v)
                 g.profile(1)

@@ -223,17 +223,6 @@ std::vector<double> lsolve(std::vector<std::vector<double>> A, std::vector<doubl
     return x;
 }
 
-struct Batch {
-    fp_ctx* c;
-    int n = 0, nch = 0;
-    size_t nvec = 0;
-    int *d_ch0 = nullptr, *d_ch1 = nullptr, *d_cptr = nullptr;
-    double* part = nullptr;  // [K][nch]
-    double* cbuf = nullptr;  // [K][n] per-case results
-    int* d_mask = nullptr;
-    std::vector<double> h;   // host mirror of cbuf
-};
-
 // the chunk table of the cases' element ranges and the reduction buffers (on first use)
 int batch_prepare(fp_ctx* c, int kmax) {
     const int n = c->n_cases;

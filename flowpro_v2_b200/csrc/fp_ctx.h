@@ -89,14 +89,12 @@ struct fp_ctx {
     // coupling e with its neighbour over face k (L for lower-ranked, U for higher-ranked)
     double* d_iluF64 = nullptr;
     float* d_iluF32 = nullptr;
-    int* d_rank = nullptr;        // DOF position of each element
     int* d_lvlF = nullptr;        // elements grouped by forward level (lower neighbours first)
     int* d_opPtr = nullptr;       // factorisation program per element
     int4* d_ops = nullptr;
-    std::vector<int> lvlF_ptr, lvlB_ptr;
+    std::vector<int> lvlF_ptr;
     bool ilu_built = false;
     int ilu_prec = -1;
-    int4* d_nbLow = nullptr;      // per element: neighbour over face f if it is lower-ranked, else -1
     int* d_swEl = nullptr;        // sweep program: element at position v (forward levels, then backward levels)
     int4* d_swNb = nullptr;       // sweep program: neighbours multiplied at position v (lower, then upper; -1 none)
     unsigned* d_iluFlags = nullptr;  // abort word, sweep status word, then [nElem] factorisation row flags

@@ -315,7 +315,8 @@ int ilu_build(fp_ctx* c) {
     };
     std::vector<int> elF, elB;
     group(levF, elF, c->lvlF_ptr);
-    group(levB, elB, c->lvlB_ptr);
+    std::vector<int> ptrB;
+    group(levB, elB, ptrB);
     std::vector<int4> nbLow(nE), nbUp(nE);
     for (int i = 0; i < nE; i++) {
         int lo[4] = {-1, -1, -1, -1}, up[4] = {-1, -1, -1, -1};
@@ -371,9 +372,8 @@ int ilu_build(fp_ctx* c) {
     }
     opPtr[nE] = (int)ops.size();
     int rc;
-    if ((rc = ialloc(c, &c->d_rank, nE)) || (rc = ialloc(c, &c->d_lvlF, nE)) ||
-        (rc = ialloc(c, &c->d_opPtr, nE + 1)) || (rc = ialloc(c, &c->d_ops, ops.size())) ||
-        (rc = ialloc(c, &c->d_nbLow, nE)) || (rc = ialloc(c, &c->d_swEl, 2 * (size_t)nE)) ||
+    if ((rc = ialloc(c, &c->d_lvlF, nE)) || (rc = ialloc(c, &c->d_opPtr, nE + 1)) ||
+        (rc = ialloc(c, &c->d_ops, ops.size())) || (rc = ialloc(c, &c->d_swEl, 2 * (size_t)nE)) ||
         (rc = ialloc(c, &c->d_swNb, 2 * (size_t)nE)) ||
         (rc = ialloc(c, &c->d_iluFlags, 2 + (size_t)nE)) || (rc = ialloc(c, &c->d_ilu_pub, 4 * (size_t)nE * c->nc)) ||
         (rc = ialloc(c, &c->d_ilu_sing, (size_t)nE)))
@@ -382,9 +382,9 @@ int ilu_build(fp_ctx* c) {
     auto up = [&](void* d, const void* hsrc, size_t bytes) {
         return cuda_check(c, cudaMemcpyAsync(d, hsrc, bytes, cudaMemcpyHostToDevice, s), "upload");
     };
-    if ((rc = up(c->d_rank, rank.data(), nE * sizeof(int))) || (rc = up(c->d_lvlF, elF.data(), nE * sizeof(int))) ||
+    if ((rc = up(c->d_lvlF, elF.data(), nE * sizeof(int))) ||
         (rc = up(c->d_opPtr, opPtr.data(), (nE + 1) * sizeof(int))) ||
-        (rc = up(c->d_ops, ops.data(), ops.size() * sizeof(int4))) || (rc = up(c->d_nbLow, nbLow.data(), nE * sizeof(int4))) ||
+        (rc = up(c->d_ops, ops.data(), ops.size() * sizeof(int4))) ||
         (rc = up(c->d_swEl, swEl.data(), 2 * (size_t)nE * sizeof(int))) ||
         (rc = up(c->d_swNb, swNb.data(), 2 * (size_t)nE * sizeof(int4))) ||
         (rc = cuda_check(c, cudaMemsetAsync(c->d_iluFlags, 0, (2 + (size_t)nE) * sizeof(unsigned), s), "memset")) ||
@@ -492,21 +492,19 @@ void ilu_release(fp_ctx* c) {
     c->ilu_prec = -1;
     c->d_iluF64 = nullptr;
     c->d_iluF32 = nullptr;
-    c->d_rank = c->d_lvlF = c->d_opPtr = nullptr;
+    c->d_lvlF = c->d_opPtr = nullptr;
     c->d_iluFlags = nullptr;
     c->d_ilu_sing = nullptr;
     c->ilu_epoch = 0;
     c->ilu_fepoch = 0;
-    c->d_ops = c->d_nbLow = c->d_swNb = nullptr;
+    c->d_ops = c->d_swNb = nullptr;
     c->d_swEl = nullptr;
     c->d_ilu_pub = nullptr;
     c->sweep_grid = 0;
     c->ring_grid[0] = c->ring_grid[1] = 0;
     c->pub_words = fp_ctx::PUB_UNKNOWN;
     c->ring_parity = 0;
-
     c->lvlF_ptr.clear();
-    c->lvlB_ptr.clear();
 }
 
 
@@ -569,9 +567,10 @@ static int launch_register(fp_ctx* c, const T* F, const double* b, double* xx) {
                       "ILU sweeps");
 }
 
-// Elements in flight per thread block that fp_set_ilu_sweep(ctx, 2 .. 6) may ask for: a power of
-// two up to 16 for nc <= 16, 8 for nc <= 32, else 4, and no more than a budget of whole positions
-// (all 1 + nf blocks) in shared memory, 208 KB above 32 unknowns, 100 KB below, divides into
+// Elements in flight per thread block that fp_set_ilu_sweep(ctx, 2 .. 6) may ask for, as the interface
+// states it: a power of two up to 16 for nc <= 16, 8 for nc <= 32, else 4, and no more than a budget of
+// whole positions (all 1 + nf blocks) in shared memory, 208 KB above 32 unknowns, 100 KB below, divides
+// into.  The ring itself would take any number up to its groups of warps; what was refused stays refused.
 static bool sweep_groups_allowed(fp_ctx* c, int precision, int NG) {
     const int nc = c->nc, most = nc <= 16 ? 16 : nc <= 32 ? 8 : 4;
     const size_t slot = (size_t)(1 + c->hm.nf) * nc * nc * (precision == FP_PREC_FP32 ? sizeof(float) : sizeof(double));
