@@ -3,15 +3,15 @@
 // A pageable copy goes through the driver's staging buffer on one thread, which also takes the page
 // faults of a fresh destination: 38 MB (200,568 triangles of 24 unknowns) took 8.2 to 17 ms down,
 // where the link needs 0.8.  Here the chunks go through pinned staging slots while several threads copy
-// between the slots and the caller's memory, each its slice of every chunk: 2.45 ms.  Copies below
-// kLeastBytes, pinned host memory and calls that find the staging memory in use by another thread take
+// between the slots and the caller's memory, each its slice of every chunk: 2.5 ms.  Copies below
+// kLeastDown and kLeastUp, pinned host memory and calls that find the staging memory in use by another thread take
 // the plain cudaMemcpyAsync.
 //
-// The slots are small because pinning them is part of the first large copy of a program that has one
-// context at a time: 12 MB take 5.0 to 8.4 ms to allocate and 1.4 to free, 6 MB 2.7 to 5.7 and 0.9.
-// State of 38 MB down / up, ms: 6 slots of 2 MB 2.5 / 2.3, 6 of 1 MB 2.45 / 2.1, 4 of 1 MB 2.65 / 1.85, 3 of
-// 1 MB 3.0 / 1.7, 6 of 512 KB 2.8 / 1.8.  The threads exist only while the link is at work: the stream's
-// earlier work is waited for first.
+// Smaller slots were measured: 38 MB down / up, ms, 6 slots of 2 MB 2.5 / 2.3, 6 of 1 MB 2.45 / 2.1, 4 of 1 MB
+// 2.65 / 1.85, 6 of 512 KB 2.8 / 1.8; but with 1 MB (slices of 128 KB) the threads' page faults meet in the same
+// 2 MB of the destination, and 27 to 33 MB take 0.4 ms longer.  Pinning the 12 MB (5.0 to 8.4 ms, once while
+// there are contexts) is part of the first copy that is large enough.  The threads exist only while the
+// link is at work: the stream's earlier work is waited for first.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -26,9 +26,14 @@ namespace fp {
 
 namespace {
 
-constexpr size_t kSlotBytes = (size_t)1 << 20;
+constexpr size_t kSlotBytes = (size_t)2 << 20;
 constexpr int kSlots = 6;
-constexpr size_t kLeastBytes = (size_t)2 << 20;
+// Smallest copies that gain.  Below, starting the threads and their page faults in one address space cost
+// more than they save.  Five explicit steps with the state read into a new array, ms, plain and staged: 2.7
+// MB 1.10 and 1.67, 4.6 MB 1.57 and 2.35, 7.4 MB 2.05 and 2.9, 11.4 MB 2.97 and 3.6, 15.3 MB 3.7 and 4.0, 22.8 MB
+// 5.2 and 5.0, 29.2 MB 6.6 and 5.8; the copy alone from 32.5 MB, where such an array is always fresh
+// memory, 8.0 and 2.65.  Up: 16 MB 0.96 and 1.48, 27 MB 1.69 and 1.72, 32.5 MB 2.4 and 1.92, 65 MB 5.9 and 3.2.
+constexpr size_t kLeastDown = (size_t)20 << 20, kLeastUp = (size_t)32 << 20;
 constexpr unsigned kMostThreads = 8;
 
 // One staging buffer per process, held by one copy at a time, freed with the last context.
@@ -108,7 +113,7 @@ struct Copiers {
 // the copy through the staging slots; *taken false: not applicable here, nothing has been copied
 int staged_copy(fp_ctx* c, void* host, void* dev, size_t bytes, bool down, bool* taken) {
     *taken = false;
-    if (bytes < kLeastBytes || !pageable(host)) return FP_OK;
+    if (bytes < (down ? kLeastDown : kLeastUp) || !pageable(host)) return FP_OK;
     Staging& S = staging();
     std::unique_lock<std::mutex> lock(S.use, std::try_to_lock);
     if (!lock.owns_lock()) return FP_OK;
