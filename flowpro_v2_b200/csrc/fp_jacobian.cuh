@@ -15,7 +15,10 @@
 // What bounds it: the products with the basis, about NC multiply-adds a point and column, each
 // shared-memory load feeding NB of them.  Measured, ms: 86,700 tetrahedra p = 2 (50 unknowns, FP32 factor
 // storage) 38.7 -> 8.4; 8,832 triangles Spalart-Allmaras p = 2 1.24 -> 0.55; the adjoint product of 10,004
-// triangles Navier-Stokes p = 2 0.63 -> 0.16.
+// triangles Navier-Stokes p = 2 0.63 -> 0.16.  Where gradients are read only through the artificial viscosity,
+// their matrices exist only at the points that have any: 106,400 triangles Euler p = 1 with the shock sensor on,
+// none active 1.07 -> 0.82, 17 % of the elements active 1.08 -> 0.97 (0.84 before these kernels); 61,440
+// tetrahedra 4.2 -> 3.0 and 4.3 -> 3.5 (3.3).
 #pragma once
 
 namespace fp {
@@ -42,6 +45,22 @@ struct JacCfg {
     static constexpr int E = cmax(1, cmin(cmin(32, THREADS / NC), (108 * 1024 / 8) / PER));
     static constexpr size_t SMEM = (size_t)E * PER * sizeof(double);
     static constexpr int CTAS = SMEM <= 112 * 1024 ? 2 : 1;
+    // task t of points * S * NE: point, seed set s and equation m.  Where gradients are read only through the
+    // artificial viscosity, the sets s > 0 of most points have nothing to do: they come last, so that whole
+    // warps skip them.
+    static __device__ __forceinline__ void task(int t, int points, int& point, int& s, int& m) {
+        if (Mdl::kViscous || Mdl::kSource) {
+            point = t / (S * NE);
+            const int seed = t - point * S * NE;
+            s = seed / NE;
+            m = seed - s * NE;
+        } else {
+            s = t / (points * NE);
+            t -= s * points * NE;
+            point = t / NE;
+            m = t - point * NE;
+        }
+    }
 };
 
 // MODE JAC_BLOCKS: Adiag = a1 M - dR/dW and Aneigh in the field-major storage of the operator; JAC_FACTOR:
@@ -115,10 +134,13 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
     __syncthreads();
     // ------------------------------------------------------------------ faces: matrices
     for (int t = threadIdx.x; t < n * C::PF * S * NE; t += C::THREADS) {
-        const int seed = t % (S * NE), xp = t / (S * NE), x = xp / C::PF, pt = xp - x * C::PF, k = pt / NQF, p = pt - k * NQF;
-        const int s = seed / NE, mj = seed - s * NE, ee = e0 + x;
+        int xp, s, mj;
+        C::task(t, n * C::PF, xp, s, mj);
+        const int x = xp / C::PF, pt = xp - x * C::PF, k = pt / NQF, p = pt - k * NQF, ee = e0 + x;
         const int TT = M.tt[(size_t)k * ld + ee];
         const bool interior = TT > -1;
+        const double eps_e = ldg(M.eps + ee), eps_nb = interior ? ldg(M.eps + TT) : 0.0;
+        if (s > 0 && !El::needs_gradients(M, interior, eps_e, eps_nb)) continue;  // nothing reads this matrix
         const double* o = trc + (size_t)xp * C::TRF;
         constexpr int NG = GRAD ? DIM * NE : 1;
         Dual<1> WL[NE], WR[NE], dWL[NG], dWR[NG], Cc[NE], Jm[NE];
@@ -143,8 +165,7 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
         }
         double nrm[DIM], Jac, dL;
         El::face_geo(M, ee, k, nrm, Jac, dL);
-        El::template point_flux<GRAD>(M, ee, k, p, TT, nrm, dL, ldg(M.eps + ee), interior ? ldg(M.eps + TT) : 0.0, WL, WR, dWL,
-                                      dWR, Cc, Jm);
+        El::template point_flux<GRAD>(M, ee, k, p, TT, nrm, dL, eps_e, eps_nb, WL, WR, dWL, dWR, Cc, Jm);
         const double jw = Jac * ldg(M.tab + TB::o_wf + p);
         const double cip = Mdl::kViscous && (interior || Mdl::isIPFace(TT)) ? ldg(M.cip + ee) : 0.0;
         double* q = mat + (size_t)xp * C::MATF + s * NE * NE + mj;
@@ -155,12 +176,23 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
     // ------------------------------------------------------------------ faces: products with the basis
     double K[MODE == JAC_VJP ? 1 : NC];
     double gi = 0.0;
+    // the faces whose gradients' matrices exist (one bit each)
+    unsigned gradFaces = 0u;
+    if constexpr (GRAD) {
+#pragma unroll
+        for (int k = 0; k < NF; k++) {
+            const int TT = M.tt[(size_t)k * ld + e];
+            if (El::needs_gradients(M, TT > -1, ldg(M.eps + e), TT > -1 ? ldg(M.eps + TT) : 0.0)) gradFaces |= 1u << k;
+        }
+    }
     // row m of the point's matrix times what the column enters through
-    auto entry = [&](const double* q, int m, double ph, const double* dph) {
+    auto entry = [&](const double* q, int k, int m, double ph, const double* dph) {
         double a = q[m * NE + mi] * ph;
         if constexpr (GRAD) {
+            if (Mdl::kViscous || (gradFaces >> k & 1u)) {
 #pragma unroll
-            for (int d = 0; d < DIM; d++) a += q[((1 + d) * NE + m) * NE + mi] * dph[d];
+                for (int d = 0; d < DIM; d++) a += q[((1 + d) * NE + m) * NE + mi] * dph[d];
+            }
         }
         return a;
     };
@@ -179,7 +211,7 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
                 column(M.tab + TB::o_phiL + pt * NB, M.tab + TB::o_dphiL + pt * NB * DIM, ph, dph);
                 const double* q = mat + (size_t)(el * C::PF + pt) * C::MATF;
 #pragma unroll
-                for (int m = 0; m < NE; m++) gi += entry(q, m, ph, dph) * lm[(el * C::PF + pt) * NE + m];
+                for (int m = 0; m < NE; m++) gi += entry(q, pt / NQF, m, ph, dph) * lm[(el * C::PF + pt) * NE + m];
             }
         } else {
             // what the element's faces add to its neighbours' rows
@@ -199,7 +231,7 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
                     const double* phiR = M.tab + TB::o_phiR + (fc * NQF + p) * NB;
                     double a[NE];
 #pragma unroll
-                    for (int m = 0; m < NE; m++) a[m] = entry(q, m, ph, dph);
+                    for (int m = 0; m < NE; m++) a[m] = entry(q, k, m, ph, dph);
 #pragma unroll
                     for (int j = 0; j < NB; j++) {
                         const double pr = ldg(phiR + j);
@@ -225,7 +257,7 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
                 const double* q = mat + (size_t)(el * C::PF + pt) * C::MATF;
                 double a[NE];
 #pragma unroll
-                for (int m = 0; m < NE; m++) a[m] = entry(q, m, ph, dph);
+                for (int m = 0; m < NE; m++) a[m] = entry(q, pt / NQF, m, ph, dph);
 #pragma unroll
                 for (int j = 0; j < NB; j++) {
                     const double pj = ldg(phi + j);
@@ -269,8 +301,10 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
         }
         __syncthreads();
         for (int t = threadIdx.x; t < n * NQV * S * NE; t += C::THREADS) {
-            const int seed = t % (S * NE), xq = t / (S * NE), x = xq / NQV, q = xq - x * NQV;
-            const int s = seed / NE, mj = seed - s * NE, ee = e0 + x;
+            int xq, s, mj;
+            C::task(t, n * NQV, xq, s, mj);
+            const int x = xq / NQV, q = xq - x * NQV, ee = e0 + x;
+            if (s > 0 && !Mdl::kViscous && !Mdl::kSource && ldg(M.eps + ee) + M.dampConst == 0.0) continue;
             const double* o = trc + (size_t)xq * C::TRV;
             double Ji[DIM * DIM];
 #pragma unroll
@@ -304,6 +338,7 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
         }
         __syncthreads();
         if (act) {
+            const bool gradVol = GRAD && (Mdl::kViscous || Mdl::kSource || ldg(M.eps + e) + M.dampConst != 0.0);
 #pragma unroll 1
             for (int q = 0; q < NQV; q++) {
                 const double *phi = M.tab + TB::o_phi + q * NB, *dphi = M.tab + TB::o_dphi + q * NB * DIM;
@@ -313,8 +348,10 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
                 auto volume_entry = [&](int d, int m) {
                     double a = w[(d * NE + m) * NE] * ph;
                     if constexpr (GRAD) {
+                        if (gradVol) {
 #pragma unroll
-                        for (int s = 1; s < S; s++) a += w[((s * C::OUT + d) * NE + m) * NE] * dph[s - 1];
+                            for (int s = 1; s < S; s++) a += w[((s * C::OUT + d) * NE + m) * NE] * dph[s - 1];
+                        }
                     }
                     return a;
                 };
@@ -378,7 +415,12 @@ __global__ void __launch_bounds__(JacCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (JacCf
 //
 // What bounds it: the NC + 1 evaluations of the flux at each point.  A thread per element and column that
 // forms all traces itself, with 2 NC sums in local memory, measured, ms: 18,000 tetrahedra Euler p = 2
-// 8.4 -> 3.9; 50,416 triangles Navier-Stokes p = 2 3.1 -> 2.5.
+// 8.4 -> 3.9; 50,416 triangles Navier-Stokes p = 2 3.1 -> 2.5.  The artificial viscosity of an inviscid model is
+// added behind the flux, where there is any (in one evaluation the gradients of both sides stay in registers
+// across the flux): 106,400 triangles Euler p = 1 with the shock sensor on, none active 1.29 -> 1.09, 17 %
+// active 1.31 -> 1.21 (1.08 by the thread per column); 61,440 tetrahedra 4.7 -> 3.0 and 4.8 -> 3.5 (3.2).
+// Viscous tetrahedra keep one thread block per SM: with two they spill 5 KB a thread (61,440 of 20 unknowns
+// 6.95 -> 6.5, 18,000 of 50 7.8 -> 6.4).
 template <class Mdl, int DIM, int ORDER, bool GRAD>
 struct FdCfg {
     using El = Element<Mdl, DIM, ORDER>;
@@ -398,7 +440,7 @@ struct FdCfg {
     static constexpr int E = cmax(1, cmin(32, cmin(THREADS * ITEMS_MAX / (COLS * NE), (100 * 1024 / 8) / PER)));
     static constexpr int ITEMS = (E * COLS * NE + THREADS - 1) / THREADS;
     static constexpr size_t SMEM = (size_t)E * PER * sizeof(double);
-    static constexpr int CTAS = SMEM <= 112 * 1024 ? 2 : 1;
+    static constexpr int CTAS = SMEM <= 112 * 1024 && !(Mdl::kViscous && DIM == 3) ? 2 : 1;
 };
 
 template <class Mdl, int DIM, int ORDER, bool GRAD>
@@ -409,7 +451,7 @@ __global__ void __launch_bounds__(FdCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (FdCfg<
     using TB = Tab<DIM, ORDER>;
     using GL = GeoLayout<DIM>;
     constexpr int NC = C::NC, NE = C::NE, NB = C::NB, NF = El::NF, NQF = El::NQF, NQV = El::NQV, NP = El::NP, S = C::S, E = C::E;
-    constexpr int COLS = C::COLS, SLOT = E * COLS, NG = GRAD ? DIM * NE : 1;
+    constexpr int COLS = C::COLS, SLOT = E * COLS;
     extern __shared__ __align__(16) double fp_dyn_smem[];
     double* coef = fp_dyn_smem;           // [c][element]
     double* trc = coef + E * NC;          // [point and side][equation][value, gradient][element]
@@ -460,28 +502,42 @@ __global__ void __launch_bounds__(FdCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (FdCfg<
         }
     }
     // the traces of a point with column i's perturbation: equation mi's is formed again
-    auto perturbed = [&](int pt, int x, int i, const double* phi, const double* dphi, const double* Ji, double* v, double* dv) {
+    auto perturbed = [&](auto grad, int pt, int x, int i, const double* phi, const double* dphi, const double* Ji, double* v, double* dv) {
+        constexpr bool G = decltype(grad)::value;
         const int mi = i / NB, bi = i - mi * NB;
         double pv = 0.0, pg[DIM], pd[DIM];
         if (i < NC) {
-            El::template trace_sums<GRAD>(
+            El::template trace_sums<G>(
                 phi, dphi,
                 [&](int j) {
                     const double c = coef[(mi * NB + j) * E + x];
                     return j == bi ? c + h : c;
                 },
                 pv, pg, 1);
-            if constexpr (GRAD) El::physical_gradient(Ji, pg, pd, 1);
+            if constexpr (G) El::physical_gradient(Ji, pg, pd, 1);
         }
         const double* o = trc + (size_t)(pt * NE * S) * E + x;
 #pragma unroll
         for (int m = 0; m < NE; m++) {
             v[m] = m == mi ? pv : o[m * S * E];
-            if constexpr (GRAD) {
+            if constexpr (G) {
 #pragma unroll
                 for (int d = 0; d < DIM; d++) dv[d * NE + m] = m == mi ? pd[d] : o[(m * S + 1 + d) * E];
             }
         }
+    };
+    // the gradient of the perturbed equation alone
+    auto perturbed_gradient = [&](int x, int i, const double* phi, const double* dphi, const double* Ji, double* pd) {
+        const int mi = i / NB, bi = i - mi * NB;
+        double pv, pg[DIM];
+        El::template trace_sums<true>(
+            phi, dphi,
+            [&](int j) {
+                const double c = coef[(mi * NB + j) * E + x];
+                return j == bi ? c + h : c;
+            },
+            pv, pg, 1);
+        El::physical_gradient(Ji, pg, pd, 1);
     };
     double K[C::ITEMS][NB];
 #pragma unroll
@@ -498,27 +554,52 @@ __global__ void __launch_bounds__(FdCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (FdCfg<
             if (x >= n) continue;
             const int TT = M.tt[(size_t)k * ld + e];
             const bool interior = TT > -1;
-            double Ji[GRAD ? DIM * DIM : 1], WL[NE], WR[NE], dWL[NG], dWR[NG], Cc[NE], Jm[NE];
-            if constexpr (GRAD) {
+            const double eps_e = ldg(M.eps + e), eps_nb = interior ? ldg(M.eps + TT) : 0.0;
+            double nrm[DIM], Jac, dL, Cc[NE], Jm[NE];
+            El::face_geo(M, e, k, nrm, Jac, dL);
+            // gradients in the flux itself only where it reads them; the artificial viscosity's are added
+            // behind it, in the order of the element residual, on the faces that have any: kept in registers
+            // across the flux they spill
+            constexpr bool G = Mdl::kViscous;
+            constexpr int NG = G ? DIM * NE : 1;
+            const double *phiL = M.tab + TB::o_phiL + pt * NB, *dphiL = M.tab + TB::o_dphiL + pt * NB * DIM;
+            const double *oL = trc + (size_t)(pt * NE * S) * E + x, *oR = trc + (size_t)((C::PF + pt) * NE * S) * E + x;
+            double Ji[GRAD ? DIM * DIM : 1], WL[NE], WR[NE], dWL[NG], dWR[NG];
+            auto geometry = [&] {
 #pragma unroll
                 for (int c = 0; c < DIM * DIM; c++) Ji[c] = ldg(M.geo + (size_t)(GL::JINV + c) * ld + e);
-            }
-            perturbed(pt, x, i, M.tab + TB::o_phiL + pt * NB, M.tab + TB::o_dphiL + pt * NB * DIM, Ji, WL, dWL);
+            };
+            if constexpr (G) geometry();
+            perturbed(std::bool_constant<G>{}, pt, x, i, phiL, dphiL, Ji, WL, dWL);
             if (interior) {
-                const double* o = trc + (size_t)((C::PF + pt) * NE * S) * E + x;
 #pragma unroll
                 for (int m = 0; m < NE; m++) {
-                    WR[m] = o[m * S * E];
-                    if constexpr (GRAD) {
+                    WR[m] = oR[m * S * E];
+                    if constexpr (G) {
 #pragma unroll
-                        for (int d = 0; d < DIM; d++) dWR[d * NE + m] = o[(m * S + 1 + d) * E];
+                        for (int d = 0; d < DIM; d++) dWR[d * NE + m] = oR[(m * S + 1 + d) * E];
                     }
                 }
             }
-            double nrm[DIM], Jac, dL;
-            El::face_geo(M, e, k, nrm, Jac, dL);
-            El::template point_flux<GRAD>(M, e, k, p, TT, nrm, dL, ldg(M.eps + e), interior ? ldg(M.eps + TT) : 0.0, WL, WR, dWL,
-                                          dWR, Cc, Jm);
+            El::template point_flux<G>(M, e, k, p, TT, nrm, dL, eps_e, eps_nb, WL, WR, dWL, dWR, Cc, Jm);
+            if constexpr (GRAD && !G) {
+                if (El::needs_gradients(M, interior, eps_e, eps_nb)) {
+                    const int mi = i / NB;
+                    double pd[DIM];
+                    if (i < NC) {
+                        geometry();
+                        perturbed_gradient(x, i, phiL, dphiL, Ji, pd);
+                    }
+#pragma unroll
+                    for (int m = 0; m < NE; m++) {
+                        double dWsum = 0.0;
+#pragma unroll
+                        for (int d = 0; d < DIM; d++)
+                            dWsum += ((i < NC && m == mi ? pd[d] : oL[(m * S + 1 + d) * E]) + oR[(m * S + 1 + d) * E]) / 2.0 * nrm[d];
+                        Cc[m] += El::artificial_flux(M, dL, eps_e, eps_nb, dWsum, WL[m], WR[m]);
+                    }
+                }
+            }
             const double jw = Jac * ldg(M.tab + TB::o_wf + p);
             const bool ip = Mdl::kViscous && (interior || Mdl::isIPFace(TT));
             const double cip = ip ? ldg(M.cip + e) : 0.0;
@@ -583,13 +664,26 @@ __global__ void __launch_bounds__(FdCfg<Mdl, DIM, ORDER, GRAD>::THREADS, (FdCfg<
                 double Ji[DIM * DIM], WI[NE], dWI[DIM * NE], Gr[DIM * NE], sw[NE];
 #pragma unroll
                 for (int c = 0; c < DIM * DIM; c++) Ji[c] = ldg(M.geo + (size_t)(GL::JINV + c) * ld + e);
-                perturbed(2 * C::PF + q, x, i, M.tab + TB::o_phi + q * NB, M.tab + TB::o_dphi + q * NB * DIM, Ji, WI, dWI);
-                if constexpr (!GRAD) {  // nothing reads the gradient: its coefficient is exactly zero
+                const double avc = ldg(M.eps + e) + M.dampConst;
+                const double *phi = M.tab + TB::o_phi + q * NB, *dphi = M.tab + TB::o_dphi + q * NB * DIM;
+                constexpr bool G = Mdl::kViscous || Mdl::kSource;
+                perturbed(std::bool_constant<G>{}, 2 * C::PF + q, x, i, phi, dphi, Ji, WI, dWI);
+                if constexpr (!G) {  // read by the artificial viscosity alone
 #pragma unroll
                     for (int c = 0; c < DIM * NE; c++) dWI[c] = 0.0;
+                    if (GRAD && avc != 0.0) {
+                        const double* oV = trc + (size_t)((2 * C::PF + q) * NE * S) * E + x;
+                        const int mi = i / NB;
+                        double pd[DIM];
+                        if (i < NC) perturbed_gradient(x, i, phi, dphi, Ji, pd);
+#pragma unroll
+                        for (int m = 0; m < NE; m++)
+#pragma unroll
+                            for (int d = 0; d < DIM; d++) dWI[d * NE + m] = i < NC && m == mi ? pd[d] : oV[(m * S + 1 + d) * E];
+                    }
                 }
                 const double jac = ldg(M.geo + (size_t)GL::JAC * ld + e);
-                El::volume_point(M, e, q, Ji, jac * ldg(M.tab + TB::o_w + q), ldg(M.eps + e) + M.dampConst, WI, dWI, Gr, sw);
+                El::volume_point(M, e, q, Ji, jac * ldg(M.tab + TB::o_w + q), avc, WI, dWI, Gr, sw);
                 double* o = gw + (size_t)r * C::OUT * NE * SLOT + i * E + x;
                 if constexpr (ORDER > 1) {
 #pragma unroll

@@ -245,6 +245,15 @@ struct Element {
         }
     }
 
+    // what the artificial viscosity of an interior face adds to an equation's integrand: dWsum the mean of
+    // the two sides' gradients along the normal, WL and WR as the flux has left them
+    static __device__ __forceinline__ double artificial_flux(const DevMesh& M, double dL, double eps_e, double eps_nb, double dWsum,
+                                                             double WL, double WR) {
+        const double idL = 1.0 / dL;
+        const double epsFace = 0.5 * (eps_e + eps_nb) + M.dampConst;
+        return epsFace * (dWsum + M.beta0 * (WR - WL) * idL);
+    }
+
     // the integrand of face_point from the traces WL and, on interior faces, WR (dWL, dWR with GRAD)
     template <bool GRAD, class T>
     static __device__ __forceinline__ void point_flux(const DevMesh& M, int e, int k, int p, int TT, const double* n, double dL,
@@ -314,7 +323,7 @@ struct Element {
 #pragma unroll
                     for (int d = 0; d < DIM; d++) dWsum += (dWL[NE * d + m] + dWR[NE * d + m]) / 2.0 * n[d];
                     const double epsFace = 0.5 * (eps_e + eps_nb) + M.dampConst;
-                    g += epsFace * (dWsum + M.beta0 * (WR[m] - WL[m]) * idL);
+                    g += epsFace * (dWsum + M.beta0 * (WR[m] - WL[m]) * idL);  // as artificial_flux
                 }
             }
             if constexpr (Mdl::kViscous) g += fvn[m];
